@@ -26,12 +26,12 @@ __host__ __device__ constexpr int pt_nb(int t) {
     struct Cls_##NAME {                                                                              \
         static constexpr int CI = ci, BI = bi, KI = ki, NOUT = nout, LL = L;                         \
         __device__ __forceinline__ static void eri(const GPair& b, const GPair& k, const PrimSoA& p, \
-                                                   const double* t, double* o) {                     \
-            eri_##NAME(b, k, p, t, o);                                                               \
+                                                   const double* t, const LaneSplit& ls, double* o) { \
+            eri_##NAME(b, k, p, t, ls, o);                                                           \
         }                                                                                            \
         __device__ __forceinline__ static void eri32(const GPair& b, const GPair& k, const PrimSoA& p, \
-                                                     const float* t, float* o) {                     \
-            eri_##NAME##_f32(b, k, p, t, o);                                                         \
+                                                     const float* t, const LaneSplit& ls, float* o) { \
+            eri_##NAME##_f32(b, k, p, t, ls, o);                                                     \
         }                                                                                            \
     };
 
@@ -159,15 +159,74 @@ struct ClassStats {
     unsigned long long scattered, prim, fp32;
 };
 
-struct NDArgs {
-    const uint2* quartets;  // this class's list: FP64 entries, then FP32 entries
-    int n;                  // number of quartets to process (ncls == nullptr)
-    // Device-side counts [2 * NCLS] (FP64, FP32 per class) written by the
-    // screen; when set, the count is ncls[2*cls+prec] and the FP32 entries
-    // start after the class's ncls[2*cls] FP64 entries, so the launch needs
-    // no host round trip and can be captured in a CUDA graph.
-    const unsigned long long* ncls;
+// One screening sub-class: the candidates of quartet class `cls` whose bra
+// pairs come from one primitive-count group of the active bra list and ket
+// pairs from one group of the ket list, so that every quartet in the
+// compacted sub-list runs its primitive loops with the same trip counts.
+struct ScreenSub {
+    long long start;   // first padded candidate index
+    long long ncand;   // candidates (unpadded)
+    int cls;
+    int same;          // one group against itself: pairs i > j only
+    int b0, nbra;      // bra range in the active list
+    int k0, nket;      // ket range
+    int npb, npk;      // primitives of the bra and ket pairs
+    // filled on the device by k_offsets, FP64 and FP32 entries:
+    long long off[2];  // write offsets (second pass)
+    int unit[2];       // first work unit within the class's list (see Unit)
+    int lgb[2], lgk[2];  // log2 of the lanes over the bra and ket primitives
+};
+
+// Work unit of a class list: one warp's share, 32 / 2^(lgb + lgk) quartets of
+// one sub-class, each spread over 2^(lgb + lgk) lanes that split its
+// primitive loops.  A quartet of two six-fold contracted s pairs runs 1296
+// primitive quartets: one thread per quartet made that one thread's serial
+// chain the time of the whole kernel for a small molecule (benzene SS|SS:
+// 255 us at 66 blocks).
+struct Unit {
+    int t;             // entry within the class's list of this precision
+    bool store;        // this lane writes the quartet's results
+    uint2 q;           // (bra, ket)
+    LaneSplit ls;
+};
+
+struct UnitList {
+    const ScreenSub* subs;             // the sub-class table
+    const unsigned long long* cnt;     // [2 * nsub] entries per sub-class (FP64, FP32)
+    const unsigned long long* ncls;    // [2 * NCLS] entries per class
+    const int* nunit;                  // [2 * NCLS] work units per class
+    int sub0, sub1;                    // sub-classes of this class
+    long long coff;                    // first entry of this class in the quartet buffer
+    const uint2* quartets;             // the whole quartet buffer
     int cls, prec;
+};
+
+// Unit u of the list: false past the end.  The lanes without a quartet (the
+// tail of a sub-class) repeat the sub-class's last one and do not store.
+__device__ __forceinline__ bool unit_of(const UnitList& L, int u, Unit& w) {
+    const int p = L.prec;
+    if (u >= L.nunit[2 * L.cls + p]) return false;
+    int lo = L.sub0, hi = L.sub1 - 1;  // last sub-class whose first unit is <= u
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (L.subs[mid].unit[p] <= u) lo = mid;
+        else hi = mid - 1;
+    }
+    const ScreenSub& S = L.subs[lo];
+    const int lgb = S.lgb[p], lgk = S.lgk[p], lg = lgb + lgk, lane = threadIdx.x & 31;
+    const int n = (int)L.cnt[2 * lo + p];
+    const int i = ((u - S.unit[p]) << (5 - lg)) + (lane >> lg);
+    const int g = lane & ((1 << lg) - 1);
+    const long long at = S.off[p] + (i < n ? i : n - 1);
+    w.q = L.quartets[at];
+    w.t = (int)(at - L.coff - (p ? (long long)L.ncls[2 * L.cls] : 0));
+    w.store = i < n && g == 0;
+    w.ls = LaneSplit{g >> lgk, 1 << lgb, g & ((1 << lgk) - 1), 1 << lgk, 1 << lg};
+    return true;
+}
+
+struct NDArgs {
+    UnitList list;
     const GPair* bra;
     const GPair* ket;
     PrimSoA prims;
@@ -218,31 +277,23 @@ static_assert(RB_THREADS * RB_SCALE == ND_THREADS, "role blocks tile a scratch t
 template <class C, bool F32>
 __global__ void __launch_bounds__(ND_THREADS) k_nondiag(NDArgs a) {
     using Real = typename std::conditional<F32, float, double>::type;
+    const int u0 = blockIdx.x * (ND_THREADS / 32);
+    if (u0 >= a.list.nunit[2 * a.list.cls + a.list.prec]) return;  // idle block of a captured grid
     __shared__ Real sboys[BOYS_BLK];
     if constexpr (F32) stage_boys<C::LL>(sboys, a.boysf);
     else stage_boys<C::LL>(sboys, a.boys);
     constexpr int NA = pt_na(C::BI), NB = pt_nb(C::BI), NC = pt_na(C::KI), ND = pt_nb(C::KI);
     static_assert(NA * NB * NC * ND == C::NOUT, "class size");
     unsigned long long nsc = 0, npr = 0;
-    const int stride = gridDim.x * blockDim.x;
-    int n = a.n;
-    const uint2* quartets = a.quartets;
-    if (a.ncls) {
-        n = (int)a.ncls[2 * a.cls + a.prec];
-        if (a.prec) quartets += a.ncls[2 * a.cls];
-    }
-    // every thread runs the same number of loop trips so the warp-level
-    // statistics reduction below sees all 32 lanes
-    const int trips = (n + stride - 1) / stride;
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int it = 0; it < trips; ++it, t += stride) {
-        if (t >= n) continue;
-        const uint2 q = quartets[t];
-        const GPair bra = a.bra[q.x];
-        const GPair ket = a.ket[q.y];
+    const int warps = gridDim.x * (ND_THREADS / 32);
+    Unit w;
+    for (int u = u0 + (threadIdx.x >> 5); unit_of(a.list, u, w); u += warps) {
+        const GPair bra = a.bra[w.q.x];
+        const GPair ket = a.ket[w.q.y];
         Real e[C::NOUT];
-        if constexpr (F32) C::eri32(bra, ket, a.prims, sboys, e);
-        else C::eri(bra, ket, a.prims, sboys, e);
+        if constexpr (F32) C::eri32(bra, ket, a.prims, sboys, w.ls, e);
+        else C::eri(bra, ket, a.prims, sboys, w.ls, e);
+        if (!w.store) continue;
         npr += (unsigned long long)(bra.np * ket.np);
         Real mx = 0;
 #pragma unroll
@@ -269,24 +320,26 @@ struct DiagArgs {
     double thr;
 };
 
+// The density screen of the diagonal builder (fock_build_diag.f90:20-21).
+__device__ __forceinline__ bool diag_screened(const GPair& pr, double sw, const double* md, int nsh, double thr) {
+    const double mv = fmax(md[pr.sa * nsh + pr.sb],
+                           fmax(0.25 * md[pr.sb * nsh + pr.sb], 0.25 * md[pr.sa * nsh + pr.sa]));
+    return sw * sw * mv < thr;
+}
+
 // Shell pairs with themselves, (ab|ab): fock_build_initial_diag.f90 (MODE 0)
-// and fock_build_diag.f90 (MODE 1).
+// and fock_build_diag.f90 (MODE 1).  One warp per pair: its lanes split the
+// np^2 primitive quartets (up to 1296), 4 over the bra and 8 over the ket.
 template <class C, int MODE>
 __global__ void __launch_bounds__(ND_THREADS) k_diag(DiagArgs a) {
-    __shared__ double sboys[BOYS_BLK];
-    stage_boys<C::LL>(sboys, a.boys);
     constexpr int NA = pt_na(C::BI), NB = pt_nb(C::BI);
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * (ND_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= a.n) return;
     const GPair pr = a.pairs[t];
-    if (MODE == 1) {
-        const double mv = fmax(a.md[pr.sa * a.nsh + pr.sb],
-                               fmax(0.25 * a.md[pr.sb * a.nsh + pr.sb], 0.25 * a.md[pr.sa * a.nsh + pr.sa]));
-        const double sw = a.schw[t];
-        if (sw * sw * mv < a.thr) return;  // fock_build_diag.f90:20-21
-    }
+    if (MODE == 1 && diag_screened(pr, a.schw[t], a.md, a.nsh, a.thr)) return;
     double e[C::NOUT];
-    C::eri(pr, pr, a.prims, sboys, e);
+    C::eri(pr, pr, a.prims, a.boys + (size_t)C::LL * BOYS_BLK, LaneSplit{lane >> 3, 4, lane & 7, 8, 32}, e);
+    if (lane) return;
     if (MODE == 0) {
         double mx = 0;
 #pragma unroll
@@ -333,7 +386,31 @@ struct StagedArgs {
     double* schw;          // per pair (MODE 0 writes, MODE 1 reads)
     const double* md;      // nsh x nsh density maxima
     int nsh;
+    // one launch per stage (gridDim.y = roles): the class's work units, or
+    // with list.subs null one quartet per unit (the diagonal builders)
+    UnitList list;
 };
+
+// Unit u of a one-launch stage: false past the end.
+__device__ __forceinline__ bool next_unit(const StagedArgs& a, int u, Unit& w) {
+    if (a.list.subs) {
+        if (!unit_of(a.list, u, w)) return false;
+        // entries of other chunks: not stored (a unit may span two chunks)
+        const long long t = w.t - a.q0;
+        w.store = w.store && t >= 0 && t < a.n;
+        w.t = (int)t;
+        return true;
+    }
+    // diagonal builders: two pairs per warp, their at most 9 x 9 primitive
+    // quartets over 4 x 4 lanes
+    if (2 * u >= a.n) return false;
+    const int lane = threadIdx.x & 31, g = lane & 15, i = 2 * u + (lane >> 4);
+    w.t = i < a.n ? i : a.n - 1;
+    w.q = a.quartets[a.q0 + w.t];
+    w.store = i < a.n && g == 0;
+    w.ls = LaneSplit{g >> 2, 4, g & 3, 4, 16};
+    return true;
+}
 
 // Quartets of this chunk: a.n, or with device-side counts the part of the
 // list left after q0, at most a.n.
@@ -775,35 +852,72 @@ __global__ void __launch_bounds__(ND_THREADS, scatg_minb(S == 0 ? NB : NA, NC, N
     }
 }
 
-// Diagonal builders of a staged class (quartets (ab|ab), one per pair):
+// Small chunks: one warp per quartet, its block in shared memory and the
+// block elements over the lanes (scatter_lanes).  The one-thread scatter is a
+// serial chain of 100-625 row loads; at a few hundred quartets that chain is
+// the kernel's time (25-100 us), while this form takes a few us.  It reads
+// each element six times from shared memory, so chunks that fill the SMs keep
+// the one-thread and grouped forms.
+constexpr int WPB = ND_THREADS / 32;  // quartets per block
+template <int NA, int NB, int NC, int ND, typename E>
+__global__ void __launch_bounds__(ND_THREADS) k_scatter_warp(StagedArgs a) {
+    constexpr int NOUT = NA * NB * NC * ND;
+    __shared__ double sw[WPB][scatter_dens(NA, NB, NC, ND)];
+    __shared__ E se[WPB][NOUT];
+    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cnt = staged_count(a);
+    unsigned long long nsc = 0, npr = 0;
+    for (int t = blockIdx.x * WPB + wp; t < cnt; t += gridDim.x * WPB) {  // whole warps
+        __syncwarp();  // the previous quartet's block has been read
+        const E* __restrict__ src = reinterpret_cast<const E*>(a.out) + tcol(t, NOUT);
+        for (int i = lane; i < NOUT; i += 32) se[wp][i] = src[(size_t)i * TQ];
+        double m = 0.0;
+        const double* __restrict__ mxc = a.mx + tcol(t, a.nroles);
+        for (int r = lane; r < a.nroles; r += 32) m = fmax(m, mxc[r * TQ]);
+        const uint2 q = staged_quartet(a, t);
+        const GPair bra = a.bra[q.x];
+        const GPair ket = a.ket[q.y];
+        npr += bra.np * ket.np;
+        if (!__any_sync(0xffffffffu, !(m < a.thr))) continue;  // fock_build_non_diag.f90:69
+        ++nsc;
+        const double s = (bra.sa == bra.sb ? 0.5 : 1.0) * (ket.sa == ket.sb ? 0.5 : 1.0);
+        scatter_lanes<NA, NB, NC, ND>(se[wp], sw[wp], s, bra, ket, a.P, a.G, a.nb, a.jonly != 0, lane, 32);
+    }
+    if (a.stats && lane == 0 && npr) {
+        atomicAdd(&a.stats->prim, npr);
+        if (nsc) atomicAdd(&a.stats->scattered, nsc);
+        if (nsc && a.f32) atomicAdd(&a.stats->fp32, nsc);
+    }
+}
+
+// Diagonal builders of a staged class (quartets (ab|ab), one warp per pair):
 // MODE 0 writes the Schwarz factor sqrt(max|e|) (fock_build_initial_diag),
 // MODE 1 applies the density screen schw^2 max(D_ab, D_aa/4, D_bb/4) < thr
 // (fock_build_diag.f90:20-21); both skip elements with |e| <= 1e-10 and
 // scatter with the weight (bra perms)^2/8.
 template <int NA, int NB, int MODE>
 __global__ void __launch_bounds__(ND_THREADS) k_scatter_diag(StagedArgs a) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int NOUT = NA * NB * NA * NB;
+    __shared__ double sw[WPB][scatter_dens(NA, NB, NA, NB)], se[WPB][NOUT];
+    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = blockIdx.x * WPB + wp;
     if (t >= staged_count(a)) return;
     const uint2 q = staged_quartet(a, t);
     const GPair pr = a.bra[q.x];
     if (MODE == 0) {
         double m = 0.0;
         for (int r = 0; r < a.nroles; ++r) m = fmax(m, a.mx[tcol(t, a.nroles) + r * TQ]);
-        a.schw[q.x] = sqrt(m);
-    } else {
-        const double mv = fmax(a.md[pr.sa * a.nsh + pr.sb],
-                               fmax(0.25 * a.md[pr.sb * a.nsh + pr.sb], 0.25 * a.md[pr.sa * a.nsh + pr.sa]));
-        const double sw = a.schw[q.x];
-        if (sw * sw * mv < a.thr) return;
+        if (lane == 0) a.schw[q.x] = sqrt(m);
+    } else if (diag_screened(pr, a.schw[q.x], a.md, a.nsh, a.thr)) {
+        return;
     }
-    double* e = a.out + tcol(t, NA * NB * NA * NB);
-#pragma unroll 1
-    for (int i = 0; i < NA * NB * NA * NB; ++i) {
-        const double v = e[(size_t)i * TQ];
-        if (!(fabs(v) > INTTHRESH)) e[(size_t)i * TQ] = 0.0;  // element skip
+    const double* __restrict__ src = a.out + tcol(t, NOUT);
+    for (int i = lane; i < NOUT; i += 32) {
+        const double v = src[(size_t)i * TQ];
+        se[wp][i] = fabs(v) > INTTHRESH ? v : 0.0;  // element skip
     }
     const double f = pr.sa == pr.sb ? 1.0 : 2.0;
-    scatter_strided<NA, NB, NA, NB>(e, TQ, f * f / 8.0, pr, pr, a.P, a.G, a.nb, false);
+    scatter_lanes<NA, NB, NA, NB>(se[wp], sw[wp], f * f / 8.0, pr, pr, a.P, a.G, a.nb, false, lane, 32);
 }
 
 typedef void (*NDKernel)(NDArgs);
@@ -819,8 +933,6 @@ struct ClassKernels {
     int mode;
     NDKernel nd64, nd32;
     DiagKernel diag0, diag1;  // only for classes (X|X)
-    int nd_threads, nd_qpb;   // block size and quartets per block
-    int dg_threads, dg_ppb;   // block size and pairs per block (diag)
     int nacc, nrole_a, nrole_b;
     int nrole_b32;            // output roles of the FP32 chunks (staged2: larger roles)
     int nrole_a32;            // accumulator roles of the FP32 chunks (staged3: larger groups)
@@ -829,12 +941,14 @@ struct ClassKernels {
     int scat_smem;                // dynamic shared memory of scat (bytes)
     StagedKernel scat32;          // scatter of FP32 chunks (float rows), or nullptr
     int scat32_smem;
+    StagedKernel scatw, scatw32;  // small chunks: one warp per quartet
     // grouped scatter (four lanes per quartet) where a bra shell has four
     // functions, else nullptr
     StagedKernel scatg, scatg32;
     int scatg_smem, scatg32_smem;
     int grp64, grp32;             // the grouped scatter is the default for FP64 / FP32 chunks
-    // every role of a stage in one launch (gridDim.y = roles), for small chunks
+    // every role of a stage in one launch (gridDim.y = roles), for small
+    // chunks; the primitive-loop stages (ma, and mb of mode 1) run on work units
     StagedKernel ma64, ma32;      // stage-A roles (staged3)
     StagedKernel mb64, mb32;      // output / HRR roles
     int bi, ki, L, nout;

@@ -316,7 +316,7 @@ class ClassGen:
         w(f"    {ft} " + ", ".join(f"{n} = 0" for n in acc.values()) + ";")
         w("    const double Ax = bra.A[0], Ay = bra.A[1], Az = bra.A[2];")
         w("    const double Cx = ket.A[0], Cy = ket.A[1], Cz = ket.A[2];")
-        w("    for (int ib = 0; ib < bra.np; ++ib) {")
+        w("    for (int ib = ls.ib; ib < bra.np; ib += ls.db) {")
         w("        const GPrim pb = load_prim(prims, bra.p0 + ib * bra.ps);")
         w(f"        const {ft} p = {cv('pb.p')};")
         w(f"        const {ft} PA0 = {cv('pb.P[0] - Ax')}, PA1 = {cv('pb.P[1] - Ay')}, PA2 = {cv('pb.P[2] - Az')};")
@@ -328,7 +328,7 @@ class ClassGen:
             wt = self.bra_combos[bi][2]
             expr = " * ".join(cv(f"pb.w{x}") for x in wt) if wt else "1"
             w(f"        const {ft} wb{bi} = {expr};")
-        w("        for (int ik = 0; ik < ket.np; ++ik) {")
+        w("        for (int ik = ls.ik; ik < ket.np; ik += ls.dk) {")
         w("            const GPrim pk = load_prim(prims, ket.p0 + ik * ket.ps);")
         w(f"            const {ft} q = {cv('pk.p')};")
         one = "1.0" if dbl else "1.0f"
@@ -381,6 +381,11 @@ class ClassGen:
                 wexp.append(f"wk{ki}")
             w(f"            {nm} += {' * '.join(wexp + [src])};")
         w("        }")
+        w("    }")
+        # the lanes that share the quartet sum their accumulators (no code
+        # where the split is the constant one_lane())
+        w("    for (int o = 1; o < ls.n; o <<= 1) {")
+        out += [f"        {nm} = lane_add({nm}, o);" for nm in acc.values()]
         w("    }")
         nbracket = sum(line.count(" - r") for line in em.lines)
         return out, acc, {"vrr": vrr.nops, "bracket": nbracket, "acc": len(acc), "order": vrr.order}
@@ -469,7 +474,7 @@ class ClassGen:
         out = [f"// ({self.A}{self.B}|{self.C}{self.D}) outputs {outs[0]}..{outs[-1]} ({len(outs)}): L={self.L}, "
                f"{vst['acc']} accumulators, VRR {vst['vrr']} terms ({vst['order']}-first)",
                f"__device__ __forceinline__ void {fname}(const GPair& bra, const GPair& ket,",
-               f"    const PrimSoA& prims, const {ft}* __restrict__ btab, {ft}* __restrict__ out)",
+               f"    const PrimSoA& prims, const {ft}* __restrict__ btab, const LaneSplit& ls, {ft}* __restrict__ out)",
                "{"]
         out += vlines + hlines
         out += [f"    out[{r}] = {v};" for r, v in enumerate(vals)]
@@ -484,11 +489,13 @@ class ClassGen:
         out = [f"// ({self.A}{self.B}|{self.C}{self.D}) accumulators ({len(keys)}): VRR {vst['vrr']} terms "
                f"({vst['order']}-first)",
                f"__device__ __forceinline__ void {fname}(const GPair& bra, const GPair& ket,",
-               f"    const PrimSoA& prims, const {ft}* __restrict__ btab, {ft}* __restrict__ dst, "
-               f"size_t stride)",
+               f"    const PrimSoA& prims, const {ft}* __restrict__ btab, const LaneSplit& ls, {ft}* __restrict__ dst, "
+               f"size_t stride, bool store)",
                "{"]
         out += vlines
-        out += [f"    dst[{k} * stride] = {acc[key]};" for k, key in enumerate(keys)]
+        out.append("    if (store) {")
+        out += [f"        dst[{k} * stride] = {acc[key]};" for k, key in enumerate(keys)]
+        out.append("    }")
         out.append("}")
         return "\n".join(out), vst
 
@@ -631,16 +638,39 @@ def acc_groups(g: "ClassGen", group: int = ACC_GROUP):
 
 
 def merged_kernel(kname: str, bodies: List[str], minb: int = 2) -> str:
-    """All roles of one stage in one launch: block row blockIdx.y runs role
-    blockIdx.y (every thread of a block runs the same role).  Used for small
-    chunks, where one launch per role would leave most SMs idle and the
+    """All roles of one HRR stage in one launch: block row blockIdx.y runs
+    role blockIdx.y (every thread of a block runs the same role).  Used for
+    small chunks, where one launch per role would leave most SMs idle and the
     launches themselves would set the time."""
-    cases = "\n".join(f"        case {r}: {b}_body(a); break;" for r, b in enumerate(bodies))
+    cases = "\n".join(f"            case {r}: {b}_body(a, t); break;" for r, b in enumerate(bodies))
     return f"""
 __global__ void __launch_bounds__(RB_THREADS, {minb} * RB_SCALE) {kname}(StagedArgs a) {{
-    switch (blockIdx.y) {{
+    const int n = staged_count(a);
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {{
+        switch (blockIdx.y) {{
 {cases}
-        default: break;
+            default: break;
+        }}
+    }}
+}}"""
+
+
+def unit_kernel(kname: str, bodies: List[str], minb: int = 2) -> str:
+    """All roles of one primitive-loop stage in one launch, one warp per work
+    unit: block row blockIdx.y runs role blockIdx.y on the units of the class
+    (see Unit in common.cuh), whose quartets are spread over several lanes
+    where they have many primitives."""
+    cases = "\n".join(f"            case {r}: {b}_unit(a, w); break;" for r, b in enumerate(bodies))
+    return f"""
+__global__ void __launch_bounds__(RB_THREADS, {minb} * RB_SCALE) {kname}(StagedArgs a) {{
+    if (a.list.subs && staged_count(a) == 0) return;  // a chunk past the end of the list
+    Unit w;
+    for (int u = blockIdx.x; next_unit(a, u, w); u += gridDim.x) {{
+        if (!__any_sync(0xffffffffu, w.store)) continue;  // a unit of other chunks
+        switch (blockIdx.y) {{
+{cases}
+            default: break;
+        }}
     }}
 }}"""
 
@@ -697,10 +727,8 @@ def class_source(ci: int, bi: int, ki: int):
         reg.append(f"    k->mode = 0;")
         reg.append(f"    k->nd64 = k_nondiag<Cls_{g.tag}, false>;")
         reg.append(f"    k->nd32 = k_nondiag<Cls_{g.tag}, true>;")
-        reg.append(f"    k->nd_threads = ND_THREADS;\n    k->nd_qpb = ND_THREADS;")
         if bi == ki:
             reg.append(f"    k->diag0 = k_diag<Cls_{g.tag}, 0>;\n    k->diag1 = k_diag<Cls_{g.tag}, 1>;")
-            reg.append(f"    k->dg_threads = ND_THREADS;\n    k->dg_ppb = ND_THREADS;")
         info.update(roles=1, role_sizes=[g.nout], role_outs=[roles[0]], acc_groups=[])
     elif len(roles) <= prm["max_roles2"]:
         mode = "staged2"
@@ -728,12 +756,25 @@ __device__ __forceinline__ void {kname}_body(const StagedArgs& a) {{
     const GPair bra = a.bra[q.x];
     const GPair ket = a.ket[q.y];
     {real} e[{len(outs)}];
-    {fname}(bra, ket, a.prims, sboys, e);
+    {fname}(bra, ket, a.prims, sboys, one_lane(), e);
     double mx = 0.0;
     // this quartet's column of the chunk's output tile (FP32 chunks keep FP32 rows)
     {real}* out = reinterpret_cast<{real}*>(a.out) + tcol(t, {g.nout});
 {stores}
     a.mx[tcol(t, {nroles_of(f32)}) + {r} * TQ] = mx;
+}}
+__device__ __forceinline__ void {kname}_unit(const StagedArgs& a, const Unit& w) {{
+    const {real}* __restrict__ sboys = {tab} + (size_t){g.L} * BOYS_BLK;
+    const GPair bra = a.bra[w.q.x];
+    const GPair ket = a.ket[w.q.y];
+    {real} e[{len(outs)}];
+    {fname}(bra, ket, a.prims, sboys, w.ls, e);
+    if (w.store) {{
+        double mx = 0.0;
+        {real}* out = reinterpret_cast<{real}*>(a.out) + tcol(w.t, {g.nout});
+{stores}
+        a.mx[tcol(w.t, {nroles_of(f32)}) + {r} * TQ] = mx;
+    }}
 }}
 __global__ void __launch_bounds__(RB_THREADS, {prm["minb32"] if f32 else 2} * RB_SCALE) {kname}(StagedArgs a) {{ {kname}_body(a); }}"""
 
@@ -745,8 +786,8 @@ __global__ void __launch_bounds__(RB_THREADS, {prm["minb32"] if f32 else 2} * RB
             code32, _ = g32.emit_role(f"{g32.name}_r{r}", outs)
             funcs.append(code32)
             kern.append(s2_kernel(f"k_s2f_{g.tag}_r{r}", f"eri_{g.tag}_f32_r{r}", outs, r, True))
-        kern.append(merged_kernel(f"k_s2m_{g.tag}", [f"k_s2_{g.tag}_r{r}" for r in range(len(roles))]))
-        kern.append(merged_kernel(f"k_s2mf_{g.tag}", [f"k_s2f_{g.tag}_r{r}" for r in range(len(roles32))]))
+        kern.append(unit_kernel(f"k_s2m_{g.tag}", [f"k_s2_{g.tag}_r{r}" for r in range(len(roles))]))
+        kern.append(unit_kernel(f"k_s2mf_{g.tag}", [f"k_s2f_{g.tag}_r{r}" for r in range(len(roles32))]))
         reg.append(f"    k->mb64 = k_s2m_{g.tag};\n    k->mb32 = k_s2mf_{g.tag};")
         reg.append(f"    k->mode = 1;\n    k->nacc = 0;\n    k->nrole_a = 0;\n    k->nrole_b = {len(roles)};\n"
                    f"    k->nrole_b32 = {len(roles32)};")
@@ -757,7 +798,9 @@ __global__ void __launch_bounds__(RB_THREADS, {prm["minb32"] if f32 else 2} * RB
         reg.append(f"    k->scat = k_scatter_staged<{NA}, {NB}, {NC}, {ND}>;\n"
                    f"    k->scat_smem = scat_smem_bytes({NA}, {NB}, {NC}, {ND});\n"
                    f"    k->scat32 = k_scatter_staged<{NA}, {NB}, {NC}, {ND}, float>;\n"
-                   f"    k->scat32_smem = scat_smem_bytes({NA}, {NB}, {NC}, {ND}, 4);")
+                   f"    k->scat32_smem = scat_smem_bytes({NA}, {NB}, {NC}, {ND}, 4);\n"
+                   f"    k->scatw = k_scatter_warp<{NA}, {NB}, {NC}, {ND}, double>;\n"
+                   f"    k->scatw32 = k_scatter_warp<{NA}, {NB}, {NC}, {ND}, float>;")
         reg.append(grouped_scatter_reg(NA, NB, NC, ND, prm))
         if bi == ki:
             reg.append(f"    k->diag0 = nullptr;\n    k->diag1 = nullptr;")
@@ -791,7 +834,15 @@ __device__ __forceinline__ void {kpre}_{g.tag}_r{r}_body(const StagedArgs& a) {{
     const uint2 q = staged_quartet(a, t);
     const GPair bra = a.bra[q.x];
     const GPair ket = a.ket[q.y];
-    {fname}(bra, ket, a.prims, sboys, reinterpret_cast<{real}*>(a.acc) + tcol(t, {len(keyidx)}) + {base} * TQ, TQ);
+    {fname}(bra, ket, a.prims, sboys, one_lane(),
+            reinterpret_cast<{real}*>(a.acc) + tcol(t, {len(keyidx)}) + {base} * TQ, TQ, true);
+}}
+__device__ __forceinline__ void {kpre}_{g.tag}_r{r}_unit(const StagedArgs& a, const Unit& w) {{
+    const {real}* __restrict__ sboys = {tab} + (size_t){g.L} * BOYS_BLK;
+    const GPair bra = a.bra[w.q.x];
+    const GPair ket = a.ket[w.q.y];
+    {fname}(bra, ket, a.prims, sboys, w.ls,
+            reinterpret_cast<{real}*>(a.acc) + tcol(w.t, {len(keyidx)}) + {base} * TQ, TQ, w.store);
 }}
 __global__ void __launch_bounds__(RB_THREADS, 2 * RB_SCALE) {kpre}_{g.tag}_r{r}(StagedArgs a) {{ {kpre}_{g.tag}_r{r}_body(a); }}""")
                 base += len(gr)
@@ -804,9 +855,7 @@ __global__ void __launch_bounds__(RB_THREADS, 2 * RB_SCALE) {kpre}_{g.tag}_r{r}(
             for kname, fname, real in ((f"k_sb_{g.tag}_r{r}", f"hrr_{g.tag}_r{r}", "double"),
                                        (f"k_sbf_{g.tag}_r{r}", f"hrr_{g.tag}_f32_r{r}", "float")):
                 kern.append(f"""
-__device__ __forceinline__ void {kname}_body(const StagedArgs& a) {{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= staged_count(a)) return;
+__device__ __forceinline__ void {kname}_body(const StagedArgs& a, int t) {{
     const uint2 q = staged_quartet(a, t);
     const GPair bra = a.bra[q.x];
     const GPair ket = a.ket[q.y];
@@ -814,9 +863,12 @@ __device__ __forceinline__ void {kname}_body(const StagedArgs& a) {{
         {fname}(bra, ket, reinterpret_cast<const {real}*>(a.acc) + tcol(t, {len(keyidx)}),
                 reinterpret_cast<{real}*>(a.out) + tcol(t, {g.nout}) + {outs[0]} * TQ, TQ);
 }}
-__global__ void __launch_bounds__(RB_THREADS, RB_SCALE) {kname}(StagedArgs a) {{ {kname}_body(a); }}""")
-        kern.append(merged_kernel(f"k_sam_{g.tag}", [f"k_sa_{g.tag}_r{r}" for r in range(len(groups))]))
-        kern.append(merged_kernel(f"k_samf_{g.tag}", [f"k_saf_{g.tag}_r{r}" for r in range(len(groups32))]))
+__global__ void __launch_bounds__(RB_THREADS, RB_SCALE) {kname}(StagedArgs a) {{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < staged_count(a)) {kname}_body(a, t);
+}}""")
+        kern.append(unit_kernel(f"k_sam_{g.tag}", [f"k_sa_{g.tag}_r{r}" for r in range(len(groups))]))
+        kern.append(unit_kernel(f"k_samf_{g.tag}", [f"k_saf_{g.tag}_r{r}" for r in range(len(groups32))]))
         kern.append(merged_kernel(f"k_sbm_{g.tag}", [f"k_sb_{g.tag}_r{r}" for r in range(len(outroles))], minb=1))
         kern.append(merged_kernel(f"k_sbmf_{g.tag}", [f"k_sbf_{g.tag}_r{r}" for r in range(len(outroles))], minb=1))
         reg.append(f"    k->ma64 = k_sam_{g.tag};\n    k->ma32 = k_samf_{g.tag};\n"
@@ -833,7 +885,9 @@ __global__ void __launch_bounds__(RB_THREADS, RB_SCALE) {kname}(StagedArgs a) {{
         reg.append(f"    k->scat = k_scatter_staged<{NA}, {NB}, {NC}, {ND}>;\n"
                    f"    k->scat_smem = scat_smem_bytes({NA}, {NB}, {NC}, {ND});\n"
                    f"    k->scat32 = k_scatter_staged<{NA}, {NB}, {NC}, {ND}, float>;\n"
-                   f"    k->scat32_smem = scat_smem_bytes({NA}, {NB}, {NC}, {ND}, 4);")
+                   f"    k->scat32_smem = scat_smem_bytes({NA}, {NB}, {NC}, {ND}, 4);\n"
+                   f"    k->scatw = k_scatter_warp<{NA}, {NB}, {NC}, {ND}, double>;\n"
+                   f"    k->scatw32 = k_scatter_warp<{NA}, {NB}, {NC}, {ND}, float>;")
         reg.append(grouped_scatter_reg(NA, NB, NC, ND, prm))
         if bi == ki:
             reg.append(f"    k->diag0 = nullptr;\n    k->diag1 = nullptr;")
@@ -908,21 +962,21 @@ def main(outdir: str):
         lines.append(f"inline void host_eri_{ci}(const GPair& b, const GPair& k, const PrimSoA& p, const double* t,")
         lines.append(f"                          const float* tf, double* out, int f32) {{")
         if info["mode"] == "direct":
-            lines.append(f"    if (f32) {{ float o[{nout}]; eri_{tag}_f32(b, k, p, tf, o);")
+            lines.append(f"    if (f32) {{ float o[{nout}]; eri_{tag}_f32(b, k, p, tf, one_lane(), o);")
             lines.append(f"        for (int i = 0; i < {nout}; ++i) out[i] = o[i]; }}")
-            lines.append(f"    else eri_{tag}(b, k, p, t, out);")
+            lines.append(f"    else eri_{tag}(b, k, p, t, one_lane(), out);")
         elif info["mode"] == "staged2":
             for r, outs in enumerate(info["role_outs"]):
                 n = len(outs)
                 idx = ", ".join(map(str, outs))
                 lines.append(f"    if (!f32) {{ static const int ix[{n}] = {{{idx}}}; double o[{n}];")
-                lines.append(f"      eri_{tag}_r{r}(b, k, p, t, o);")
+                lines.append(f"      eri_{tag}_r{r}(b, k, p, t, one_lane(), o);")
                 lines.append(f"      for (int i = 0; i < {n}; ++i) out[ix[i]] = o[i]; }}")
             for r, outs in enumerate(info["role_outs32"]):
                 n = len(outs)
                 idx = ", ".join(map(str, outs))
                 lines.append(f"    if (f32) {{ static const int ix[{n}] = {{{idx}}}; float of[{n}];")
-                lines.append(f"      eri_{tag}_f32_r{r}(b, k, p, tf, of);")
+                lines.append(f"      eri_{tag}_f32_r{r}(b, k, p, tf, one_lane(), of);")
                 lines.append(f"      for (int i = 0; i < {n}; ++i) out[ix[i]] = of[i]; }}")
         else:
             nacc = sum(len(g) for g in info["acc_groups"])
@@ -930,11 +984,11 @@ def main(outdir: str):
             lines.append(f"    static float accf[{nacc}];")
             base = 0
             for r, gr in enumerate(info["acc_groups"]):
-                lines.append(f"    if (!f32) acc_{tag}_r{r}(b, k, p, t, acc + {base}, 1);")
+                lines.append(f"    if (!f32) acc_{tag}_r{r}(b, k, p, t, one_lane(), acc + {base}, 1, true);")
                 base += len(gr)
             base = 0
             for r, gr in enumerate(info["acc_groups32"]):
-                lines.append(f"    if (f32) acc_{tag}_f32_r{r}(b, k, p, tf, accf + {base}, 1);")
+                lines.append(f"    if (f32) acc_{tag}_f32_r{r}(b, k, p, tf, one_lane(), accf + {base}, 1, true);")
                 base += len(gr)
             for r, outs in enumerate(info["role_outs"]):
                 n = len(outs)
@@ -946,7 +1000,8 @@ def main(outdir: str):
         na, nb_, nc, nd = info["dims"]
         lines.append(f"inline int host_scatter_{ci}(const double* e, double s, const GPair& b, const GPair& k,")
         lines.append(f"                             const double* P, double* G, int nb, bool jonly) {{")
-        lines.append(f"    scatter_strided<{na}, {nb_}, {nc}, {nd}>(e, 1, s, b, k, P, G, nb, jonly);")
+        lines.append(f"    double w[scatter_dens({na}, {nb_}, {nc}, {nd})];")
+        lines.append(f"    scatter_lanes<{na}, {nb_}, {nc}, {nd}>(e, w, s, b, k, P, G, nb, jonly, 0, 1);")
         lines.append("    return 0;")
         lines.append("}")
     lines.append("typedef void (*HostEri)(const GPair&, const GPair&, const PrimSoA&, const double*, const float*, double*, int);")

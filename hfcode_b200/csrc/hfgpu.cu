@@ -146,20 +146,6 @@ __global__ void k_maxdm(const int* __restrict__ shtyp, const int* __restrict__ a
     md[(size_t)b * nsh + a] = m;
 }
 
-// One screening sub-class: the candidates of quartet class `cls` whose bra
-// pairs come from one primitive-count group of the active bra list and ket
-// pairs from one group of the ket list, so that every quartet in the
-// compacted sub-list runs its primitive loops with the same trip counts.
-struct ScreenSub {
-    long long start;   // first padded candidate index
-    long long ncand;   // candidates (unpadded)
-    int cls;
-    int same;          // one group against itself: pairs i > j only
-    int b0, nbra;      // bra range in the active list
-    int k0, nket;      // ket range
-    long long off[2];  // write offsets of the FP64 / FP32 entries (second pass)
-};
-
 struct ScreenArgs {
     const ScreenSub* subs;
     int nsub;
@@ -211,8 +197,6 @@ __global__ void k_screen(ScreenArgs a) {
             }
             ii = (unsigned)(S.b0 + i);
             jj = (unsigned)(S.k0 + j);
-            const int bt = 0;  // pair types are resolved through the class
-            (void)bt;
             const int2 ab = a.sh[CLS_BI[S.cls]][ii], cd = a.sh[CLS_KI[S.cls]][jj];
             const double dc = fmax(a.md[ab.x * a.nsh + ab.y], a.md[cd.x * a.nsh + cd.y]);
             double v = dc;
@@ -247,30 +231,87 @@ __global__ void k_screen(ScreenArgs a) {
 struct OffsetArgs {
     int csub[NCLS + 1];      // sub-classes of class c: [csub[c], csub[c+1])
     long long coff[NCLS];    // first entry of class c in the quartet buffer
+    float fill[NCLS][2];     // threads that fill the GPU with this class's kernel, per role (FP64, FP32)
+    int lmin[NCLS];          // fewest primitive quartets a lane is given
 };
+
+// Fewest lanes (lgb + lgk) over npb x npk primitives with at most `most`
+// primitive quartets per lane, and their best split over bra and ket.
+__device__ __forceinline__ void pick_lanes(int npb, int npk, int most, int& lgb, int& lgk) {
+    lgb = lgk = 0;
+    int best = npb * npk;
+    for (int lg = 1; lg <= 5 && best > most; ++lg)
+        for (int k = 0; k <= lg; ++k) {
+            const int b = lg - k;
+            const int c = ((npb + (1 << b) - 1) >> b) * ((npk + (1 << k) - 1) >> k);
+            if (c < best) {
+                best = c;
+                lgb = b;
+                lgk = k;
+            }
+        }
+}
+
+__device__ __forceinline__ long long warp_scan(long long v, int lane) {  // inclusive
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long x = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += x;
+    }
+    return v;
+}
 
 // Write offsets of the compacted lists from the pass-0 counts, on the device
 // so that a build needs no host round trip: per class its FP64 entries, then
 // its FP32 entries, sub-classes in order.  Also stores the per-class totals
-// that the class kernels read.  One thread per class.
+// that the class kernels read, and cuts each list into work units (see Unit):
+// a quartet is spread over as many lanes as it takes for a lane's share of
+// its primitive loops to be near the class's primitive work over the threads
+// that fill the GPU, and at least lmin.  A class that fills the GPU anyway
+// keeps one lane per quartet.  One warp per class.
 __global__ void k_offsets(OffsetArgs o, ScreenSub* __restrict__ subs, const unsigned long long* __restrict__ cnt,
-                          unsigned long long* __restrict__ ncls) {
-    const int c = threadIdx.x;
-    if (c >= NCLS) return;
-    unsigned long long n64 = 0, n32 = 0;
-    for (int k = o.csub[c]; k < o.csub[c + 1]; ++k) {
-        n64 += cnt[2 * k];
-        n32 += cnt[2 * k + 1];
+                          unsigned long long* __restrict__ ncls, int* __restrict__ nunit) {
+    const int c = blockIdx.x, lane = threadIdx.x;
+    const int k0 = o.csub[c], k1 = o.csub[c + 1];
+    long long n[2] = {0, 0};
+    double work[2] = {0.0, 0.0};
+    for (int k = k0 + lane; k < k1; k += 32)
+        for (int p = 0; p < 2; ++p) {
+            const long long m = (long long)cnt[2 * k + p];
+            n[p] += m;
+            work[p] += (double)m * (subs[k].npb * subs[k].npk);
+        }
+    for (int p = 0; p < 2; ++p)
+        for (int s = 16; s > 0; s >>= 1) {
+            n[p] += __shfl_xor_sync(0xffffffffu, n[p], s);
+            work[p] += __shfl_xor_sync(0xffffffffu, work[p], s);
+        }
+    long long at[2] = {o.coff[c], o.coff[c] + n[0]};
+    long long unit[2] = {0, 0};
+    for (int k = k0; k < k1; k += 32) {
+        const int x = k + lane;
+        for (int p = 0; p < 2; ++p) {
+            const long long m = x < k1 ? (long long)cnt[2 * x + p] : 0;
+            const double most = fmax((double)o.lmin[c], work[p] / (double)o.fill[c][p]);
+            int lgb = 0, lgk = 0;
+            if (x < k1) pick_lanes(subs[x].npb, subs[x].npk, (int)fmin(most, 1e6), lgb, lgk);
+            const int per = 32 >> (lgb + lgk);
+            const long long u = (m + per - 1) / per;
+            const long long sm = warp_scan(m, lane), su = warp_scan(u, lane);
+            if (x < k1) {
+                subs[x].off[p] = at[p] + sm - m;
+                subs[x].unit[p] = (int)(unit[p] + su - u);
+                subs[x].lgb[p] = lgb;
+                subs[x].lgk[p] = lgk;
+            }
+            at[p] += __shfl_sync(0xffffffffu, sm, 31);
+            unit[p] += __shfl_sync(0xffffffffu, su, 31);
+        }
     }
-    long long p64 = o.coff[c], p32 = o.coff[c] + (long long)n64;
-    for (int k = o.csub[c]; k < o.csub[c + 1]; ++k) {
-        subs[k].off[0] = p64;
-        subs[k].off[1] = p32;
-        p64 += (long long)cnt[2 * k];
-        p32 += (long long)cnt[2 * k + 1];
+    if (lane < 2) {
+        ncls[2 * c + lane] = (unsigned long long)(lane ? n[1] : n[0]);
+        nunit[2 * c + lane] = (int)(lane ? unit[1] : unit[0]);
     }
-    ncls[2 * c] = n64;
-    ncls[2 * c + 1] = n32;
 }
 
 // The density in shell-pair blocks: block (s1, s2) holds P[r][c] for the
@@ -376,12 +417,15 @@ struct hfgpu_handle {
     long long ccap[NCLS] = {};      // candidates per class (upper bound of its list)
     long long coff[NCLS] = {};      // class region in the quartet buffer
     long long n64[NCLS] = {}, n32[NCLS] = {};
+    int nunit[2 * NCLS] = {};       // work units of the last eager build
     cudaEvent_t ev[2 * NCLS + 2] = {};
     int nsm = 148;
     long long launches = 0;             // kernels enqueued by this handle (graph replays included)
     long long graph_launches = 0;       // kernels in the captured build
     OffsetArgs offs{};                  // sub-class ranges / list regions per class
-    unsigned long long* d_ncls = nullptr;  // [2 * NCLS] surviving quartets (FP64, FP32) per class
+    // [2 * NCLS] surviving quartets (FP64, FP32) per class, then as ints the work units
+    unsigned long long* d_ncls = nullptr;
+    long long warp_scatter = 0;         // chunks up to this many quartets use the one-warp-per-quartet scatter
     double* d_Pb = nullptr;             // density in shell-pair blocks (nb x nb)
     int* d_boff = nullptr;              // block offsets (nsh x nsh)
     int2* d_aomap = nullptr;            // per function: (shell, index within the shell)
@@ -531,12 +575,13 @@ int launch_symm(hfgpu_handle* h, double* F, const double* G = nullptr) {
 // programs, and an SM running several of them thrashes its instruction
 // cache); small chunks gain more from filling the SMs and launching less.
 bool merge_roles(const hfgpu_handle* h, const ClassKernels& K, int blocks, int roles) {
-    return K.mb64 && roles > 1 && (long long)blocks * roles <= h->merge_blocks;
+    return (long long)blocks * roles <= h->merge_blocks;
 }
 
 // Diagonal builder of a staged pair type: chunks of its pairs through the
 // class's roles and k_scatter_diag.
-int run_staged_diag(hfgpu_handle* h, int t, int mode, const double* P, double thr, double* G, const double* md) {
+int run_staged_diag(hfgpu_handle* h, int t, int mode, const double* P, double thr, double* G, const double* md,
+                    cudaStream_t stream) {
     const ClassKernels& K = CLASS_KERNELS[class_index(t, t)];
     const long long n = (long long)h->pairs[t].size();
     const size_t st = h->dstride[t];
@@ -565,51 +610,57 @@ int run_staged_diag(hfgpu_handle* h, int t, int mode, const double* P, double th
         a.schw = h->d_schw[t];
         a.md = md;
         a.nsh = h->nsh;
-        const int blocks = (m + ND_THREADS - 1) / ND_THREADS;
-        if (merge_roles(h, K, blocks, std::max(K.nrole_a, K.nrole_b))) {
-            if (K.nrole_a > 0) {
-                ++h->launches;
-                K.ma64<<<dim3(blocks * RB_SCALE, K.nrole_a), RB_THREADS, 0, h->stream>>>(a);
-                HF_CHECK(cudaGetLastError());
-            }
+        // every role of a stage in one launch, two pairs per warp in the
+        // primitive-loop stage (next_unit), then one warp per pair
+        const int blocks = (m + ND_THREADS - 1) / ND_THREADS, units = (m + 1) / 2;
+        if (K.nrole_a > 0) {
             ++h->launches;
-            K.mb64<<<dim3(blocks * RB_SCALE, K.nrole_b), RB_THREADS, 0, h->stream>>>(a);
+            K.ma64<<<dim3(units, K.nrole_a), RB_THREADS, 0, stream>>>(a);
             HF_CHECK(cudaGetLastError());
-        } else {
-            for (int r = 0; r < K.nrole_a; ++r) {
-                ++h->launches;
-                K.sa64[r]<<<blocks * RB_SCALE, RB_THREADS, 0, h->stream>>>(a);
-                HF_CHECK(cudaGetLastError());
-            }
-            for (int r = 0; r < K.nrole_b; ++r) {
-                ++h->launches;
-                K.sb64[r]<<<blocks * RB_SCALE, RB_THREADS, 0, h->stream>>>(a);
-                HF_CHECK(cudaGetLastError());
-            }
         }
         ++h->launches;
-        (mode ? K.dscat1 : K.dscat0)<<<blocks, ND_THREADS, 0, h->stream>>>(a);
+        K.mb64<<<dim3(K.nrole_a > 0 ? blocks * RB_SCALE : units, K.nrole_b), RB_THREADS, 0, stream>>>(a);
+        HF_CHECK(cudaGetLastError());
+        ++h->launches;
+        (mode ? K.dscat1 : K.dscat0)<<<(m + WPB - 1) / WPB, ND_THREADS, 0, stream>>>(a);
         HF_CHECK(cudaGetLastError());
     }
     return HFGPU_OK;
 }
 
-int launch_diag(hfgpu_handle* h, int mode, const double* P, double thr, double* G = nullptr,
-                const double* md = nullptr) {
+// Diagonal builder: the direct pair types on `s_direct`, the staged types
+// (which share one scratch) one after another on `s_staged`.
+int launch_diag(hfgpu_handle* h, int mode, const double* P, double thr, double* G, const double* md,
+                cudaStream_t s_direct, cudaStream_t s_staged) {
     for (int t = 0; t < NPT; ++t) {
         int n = (int)h->pairs[t].size();
         if (n == 0) continue;
         if (CLASS_KERNELS[class_index(t, t)].mode != 0) {
-            int rc = run_staged_diag(h, t, mode, P, thr, G ? G : h->d_G, md ? md : h->d_md);
+            int rc = run_staged_diag(h, t, mode, P, thr, G, md, s_staged);
             if (rc) return rc;
             continue;
         }
-        DiagArgs a{h->d_pairs[t], n, h->psoa, h->d_boys, h->d_schw[t], md ? md : h->d_md, h->nsh, P,
-                   G ? G : h->d_G, h->nb, thr};
-        const ClassKernels& K = CLASS_KERNELS[class_index(t, t)];
+        DiagArgs a{h->d_pairs[t], n, h->psoa, h->d_boys, h->d_schw[t], md, h->nsh, P, G, h->nb, thr};
         ++h->launches;
-        diag_kernel(t, mode)<<<(n + K.dg_ppb - 1) / K.dg_ppb, K.dg_threads, 0, h->stream>>>(a);
+        diag_kernel(t, mode)<<<(n + WPB - 1) / WPB, ND_THREADS, 0, s_direct>>>(a);
         HF_CHECK(cudaGetLastError());
+    }
+    return HFGPU_OK;
+}
+
+// The diagonal builder on the first two class streams, forked from the
+// handle's stream.  The class streams join back at the end of an
+// off-diagonal build, or here when `join` is set.
+int fork_diag(hfgpu_handle* h, int mode, const double* P, double thr, bool join) {
+    cudaStream_t s0 = h->aux[0], s1 = h->aux[h->nstreams > 1 ? 1 : 0];
+    HF_CHECK(cudaEventRecord(h->fork, h->stream));
+    HF_CHECK(cudaStreamWaitEvent(s0, h->fork, 0));
+    if (s1 != s0) HF_CHECK(cudaStreamWaitEvent(s1, h->fork, 0));
+    const int rc = launch_diag(h, mode, P, thr, h->d_G, h->d_md, s0, s1);
+    if (rc || !join) return rc;
+    for (int k = 0; k < (s1 != s0 ? 2 : 1); ++k) {
+        HF_CHECK(cudaEventRecord(h->join[k], h->aux[k]));
+        HF_CHECK(cudaStreamWaitEvent(h->stream, h->join[k], 0));
     }
     return HFGPU_OK;
 }
@@ -630,6 +681,10 @@ size_t scratch_budget_doubles() {
     }
     return mb * 1024 * 1024 / sizeof(double);
 }
+
+// Fewest primitive quartets per lane of a work unit: below these the sum of
+// the accumulators over the lanes costs more than the shorter loops save.
+constexpr int LMIN_DIRECT = 6, LMIN_STAGED = 4;
 
 // Schwarz ordering (index_sort + find_threshold) and the active pair arrays.
 int build_active(hfgpu_handle* h) {
@@ -757,6 +812,8 @@ int build_active(hfgpu_handle* h) {
                 sub.nbra = groups[bi][gb].second;
                 sub.k0 = groups[ki][gk].first;
                 sub.nket = groups[ki][gk].second;
+                sub.npb = h->act_np[bi][sub.b0];
+                sub.npk = h->act_np[ki][sub.k0];
                 sub.ncand = sub.same ? (long long)sub.nbra * (sub.nbra - 1) / 2 : (long long)sub.nbra * sub.nket;
                 if (sub.ncand == 0) continue;
                 sub.start = start;
@@ -769,6 +826,15 @@ int build_active(hfgpu_handle* h) {
         h->offs.coff[c] = qoff;
         qoff += ccap;
         h->offs.csub[c + 1] = (int)h->hsubs.size();
+        // threads that fill the GPU: 32 warps per SM of a direct kernel, 8 of
+        // the 255-register role kernels, whose roles run side by side
+        const ClassKernels& K = CLASS_KERNELS[c];
+        for (int p = 0; p < 2; ++p) {
+            const int roles = K.mode == 0 ? 1 : K.mode == 1 ? (p ? K.nrole_b32 : K.nrole_b)
+                                                            : (p ? K.nrole_a32 : K.nrole_a);
+            h->offs.fill[c][p] = (float)h->nsm * (K.mode == 0 ? 1024.f : 256.f) / (float)roles;
+        }
+        h->offs.lmin[c] = K.mode == 0 ? LMIN_DIRECT : LMIN_STAGED;
     }
     h->offs.csub[0] = 0;
     h->ntot = start;
@@ -823,10 +889,34 @@ int build_active(hfgpu_handle* h) {
     return HFGPU_OK;
 }
 
+// The work units of a class list, as the kernels take them.
+UnitList unit_list(const hfgpu_handle* h, int c, int prec) {
+    UnitList L{};
+    L.subs = h->d_subs;
+    L.cnt = h->d_cnt;
+    L.ncls = h->d_ncls;
+    L.nunit = reinterpret_cast<const int*>(h->d_ncls + 2 * NCLS);
+    L.sub0 = h->offs.csub[c];
+    L.sub1 = h->offs.csub[c + 1];
+    L.coff = h->coff[c];
+    L.quartets = h->d_q;
+    L.cls = c;
+    L.prec = prec;
+    return L;
+}
+
+// Blocks along x of a kernel that walks its list: as many as the list needs
+// where the count is on the host; in a capture, whose counts stay on the
+// device, at most `fill` (idle blocks of a grid sized by the capacity cost
+// about a nanosecond each, 0.1 ms for a class with many roles).
+unsigned walk_blocks(long long need, long long fill, bool capture) {
+    return (unsigned)std::max<long long>(1, capture ? std::min(need, fill) : need);
+}
+
 // Staged class: chunks of the quartet list through the accumulator roles
 // (mode 2), the output roles and the scatter kernel.
 int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, double thr, int jonly,
-               cudaStream_t stream, double* scratch) {
+               cudaStream_t stream, double* scratch, bool capture) {
     const ClassKernels& K = CLASS_KERNELS[c];
     const size_t st = h->stride[c];
     for (long long q0 = 0; q0 < n; q0 += (long long)st) {
@@ -861,14 +951,22 @@ int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, d
         const int blocks = (m + ND_THREADS - 1) / ND_THREADS;
         const int na = prec ? K.nrole_a32 : K.nrole_a;
         if (merge_roles(h, K, blocks, std::max(na, a.nroles))) {
-            // a small chunk: every role of a stage in one launch, side by side
+            // a small list: every role of a stage in one launch, side by side,
+            // the primitive-loop stage on the class's work units
+            a.list = unit_list(h, c, prec);
+            // a unit holds at least one quartet, so n bounds the units; two
+            // rounds of the eight resident warps per SM in a capture
+            const int nr = std::max(na, a.nroles);
+            const long long fill = (16LL * h->nsm + nr - 1) / nr;
+            const unsigned units = walk_blocks(capture ? n : h->nunit[2 * c + prec], fill, capture);
+            const unsigned hblocks = walk_blocks((long long)blocks * RB_SCALE, fill, capture);
             if (na > 0) {
                 ++h->launches;
-                (prec ? K.ma32 : K.ma64)<<<dim3(blocks * RB_SCALE, na), RB_THREADS, 0, stream>>>(a);
+                (prec ? K.ma32 : K.ma64)<<<dim3(units, na), RB_THREADS, 0, stream>>>(a);
                 HF_CHECK(cudaGetLastError());
             }
             ++h->launches;
-            (prec ? K.mb32 : K.mb64)<<<dim3(blocks * RB_SCALE, a.nroles), RB_THREADS, 0, stream>>>(a);
+            (prec ? K.mb32 : K.mb64)<<<dim3(na > 0 ? hblocks : units, a.nroles), RB_THREADS, 0, stream>>>(a);
             HF_CHECK(cudaGetLastError());
         } else {
             for (int r = 0; r < na; ++r) {
@@ -887,7 +985,10 @@ int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, d
         // everywhere it exists (2) or nowhere (0)
         const bool grp = h->grouped_scatter == 2 || (h->grouped_scatter == 1 && (prec ? K.grp32 : K.grp64));
         const StagedKernel sg = grp ? (prec ? K.scatg32 : K.scatg) : nullptr;
-        if (sg) {  // four lanes per quartet
+        if (m <= h->warp_scatter) {  // one warp per quartet
+            const unsigned wblocks = walk_blocks((m + WPB - 1) / WPB, 8LL * h->nsm, capture);
+            (prec ? K.scatw32 : K.scatw)<<<wblocks, ND_THREADS, 0, stream>>>(a);
+        } else if (sg) {  // four lanes per quartet
             const int gblocks = (int)(((long long)m * SG + ND_THREADS - 1) / ND_THREADS);
             sg<<<gblocks, ND_THREADS, prec ? K.scatg32_smem : K.scatg_smem, stream>>>(a);
         } else if (prec && K.scat32) {
@@ -909,7 +1010,7 @@ int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, d
 int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double f32cut, bool capture = false) {
     if (!h->have_schwarz) return set_err(HFGPU_ERR_STATE, "fock_build_initial_diag has not been called");
     HF_CHECK(cudaMemsetAsync(h->d_stats, 0, NCLS * sizeof(ClassStats), h->stream));
-    HF_CHECK(cudaMemsetAsync(h->d_ncls, 0, 2 * NCLS * sizeof(unsigned long long), h->stream));
+    HF_CHECK(cudaMemsetAsync(h->d_ncls, 0, 3 * NCLS * sizeof(unsigned long long), h->stream));
     const int nsub = (int)h->hsubs.size();
     for (int c = 0; c < NCLS; ++c) h->n64[c] = h->n32[c] = 0;
     if (h->ntot > 0 && nsub > 0) {
@@ -936,7 +1037,8 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
         k_screen<0><<<blocks, 256, 0, h->stream>>>(sa);  // survivors per sub-class
         HF_CHECK(cudaGetLastError());
         ++h->launches;
-        k_offsets<<<1, (NCLS + 31) / 32 * 32, 0, h->stream>>>(h->offs, h->d_subs, h->d_cnt, h->d_ncls);
+        k_offsets<<<NCLS, 32, 0, h->stream>>>(h->offs, h->d_subs, h->d_cnt, h->d_ncls,
+                                              reinterpret_cast<int*>(h->d_ncls + 2 * NCLS));
         HF_CHECK(cudaGetLastError());
         HF_CHECK(cudaMemsetAsync(h->d_cnt, 0, cbytes, h->stream));
         ++h->launches;
@@ -951,9 +1053,10 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
         HF_CHECK(cudaGetLastError());
     }
     if (!capture) {
-        unsigned long long cnt[2 * NCLS];
+        unsigned long long cnt[3 * NCLS];
         HF_CHECK(cudaMemcpyAsync(cnt, h->d_ncls, sizeof(cnt), cudaMemcpyDeviceToHost, h->stream));
         HF_CHECK(cudaStreamSynchronize(h->stream));
+        memcpy(h->nunit, cnt + 2 * NCLS, sizeof(h->nunit));
         for (int c = 0; c < NCLS; ++c) {
             h->n64[c] = (long long)cnt[2 * c];
             h->n32[c] = (long long)cnt[2 * c + 1];
@@ -993,11 +1096,7 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
         if (timed) HF_CHECK(cudaEventRecord(h->ev[2 * c], h->stream));
         if (K.mode == 0) {
             NDArgs a{};
-            a.quartets = h->d_q + h->coff[c];
-            a.n = (int)n;
-            a.ncls = h->d_ncls;
-            a.cls = c;
-            a.prec = prec;
+            a.list = unit_list(h, c, prec);
             a.bra = h->d_apairs[K.bi];
             a.ket = h->d_apairs[K.ki];
             a.prims = h->apsoa;
@@ -1009,13 +1108,13 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
             a.thr = thr;
             a.jonly = jonly;
             a.stats = h->d_stats + c;
-            long long blocks = (n + K.nd_qpb - 1) / K.nd_qpb;
-            if (capture) blocks = std::min<long long>(blocks, (long long)h->nsm * 16);  // grid-stride
+            const unsigned blocks =
+                walk_blocks(((capture ? n : h->nunit[2 * c + prec]) + WPB - 1) / WPB, 8LL * h->nsm, capture);
             ++h->launches;
-            (prec ? K.nd32 : K.nd64)<<<(int)blocks, K.nd_threads, 0, st>>>(a);
+            (prec ? K.nd32 : K.nd64)<<<blocks, ND_THREADS, 0, st>>>(a);
             HF_CHECK(cudaGetLastError());
         } else {
-            int rc = run_staged(h, c, prec, n, P, thr, jonly, st, slot);
+            int rc = run_staged(h, c, prec, n, P, thr, jonly, st, slot, capture);
             if (rc) return rc;
         }
         if (timed) {
@@ -1086,6 +1185,8 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
         // 10.8 jobs/s without merging, 14.9 at 2 x SMs, 23.9 at 8 x SMs
         h->merge_blocks = 8LL * h->nsm;
         if (const char* e = getenv("HFGPU_MERGE_BLOCKS")) h->merge_blocks = atoll(e);
+        h->warp_scatter = 16LL * h->nsm;
+        if (const char* e = getenv("HFGPU_WARP_SCATTER")) h->warp_scatter = atoll(e);
         if (const char* e = getenv("HFGPU_STREAMS")) h->nstreams = std::max(1, std::min(NSTREAM, atoi(e)));
         if (const char* e = getenv("HFGPU_SCATTER"))  // "single" / "grouped" override the per-class choice
             h->grouped_scatter = strcmp(e, "single") == 0 ? 0 : strcmp(e, "grouped") == 0 ? 2 : 1;
@@ -1103,7 +1204,7 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
     rc |= dalloc(&h->d_md, (size_t)h->nsh * h->nsh, h->stream);
     rc |= dalloc(&h->d_cnt, 2 * NCLS, h->stream);
     rc |= dalloc(&h->d_stats, NCLS, h->stream);
-    rc |= dalloc(&h->d_ncls, 2 * NCLS, h->stream);
+    rc |= dalloc(&h->d_ncls, 3 * NCLS, h->stream);
     rc |= dalloc(&h->d_Pb, nb2, h->stream);
     rc |= dalloc(&h->d_boff, (size_t)h->nsh * h->nsh, h->stream);
     rc |= dalloc(&h->d_aomap, (size_t)h->nb, h->stream);
@@ -1188,7 +1289,7 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
         }
     }
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_stats, 0, NCLS * sizeof(ClassStats), h->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_ncls, 0, 2 * NCLS * sizeof(unsigned long long), h->stream);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(h->d_ncls, 0, 3 * NCLS * sizeof(unsigned long long), h->stream);
     // the handle's own stream only: other handles' work on the device goes on
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
     if (ce != cudaSuccess) {
@@ -1273,7 +1374,7 @@ int hfgpu_fock_build_initial_diag(hfgpu_handle* h, double* f, const double* p, d
     int rc = upload_fp(h, f, p);
     if (rc) return rc;
     HF_CHECK(cudaMemsetAsync(h->d_G, 0, (size_t)h->nb * h->nb * sizeof(double), h->stream));
-    rc = launch_diag(h, 0, h->d_P, thr);
+    rc = fork_diag(h, 0, h->d_P, thr, true);
     if (rc) return rc;
     rc = launch_symm(h, h->d_F);
     if (rc) return rc;
@@ -1289,7 +1390,7 @@ int hfgpu_fock_build_diag(hfgpu_handle* h, double* f, const double* p, double th
     if (rc) return rc;
     HF_CHECK(cudaMemsetAsync(h->d_G, 0, (size_t)h->nb * h->nb * sizeof(double), h->stream));
     if ((rc = launch_maxdm(h, h->d_P))) return rc;
-    if ((rc = launch_diag(h, 1, h->d_P, thr))) return rc;
+    if ((rc = fork_diag(h, 1, h->d_P, thr, true))) return rc;
     if ((rc = launch_symm(h, h->d_F))) return rc;
     return download_f(h, f);
 }
@@ -1323,7 +1424,9 @@ static int device_build(hfgpu_handle* h, double* f_dev, const double* p_dev, dou
     int rc;
     HF_CHECK(cudaMemsetAsync(h->d_G, 0, (size_t)h->nb * h->nb * sizeof(double), h->stream));
     if ((rc = launch_maxdm(h, p_dev))) return rc;
-    if ((rc = launch_diag(h, 1, p_dev, thr_diag))) return rc;
+    // beside the screening; joined with the class streams (with per-class
+    // timing the classes run on the handle's own stream)
+    if ((rc = fork_diag(h, 1, p_dev, thr_diag, h->timing && !capture))) return rc;
     if ((rc = run_non_diag(h, p_dev, thr_non_diag, 0, fp32_cutoff, capture))) return rc;
     return launch_symm(h, f_dev);
 }
@@ -1344,7 +1447,7 @@ int hfgpu_fock_build_initial_diag_device(hfgpu_handle* h, double* f_dev, const d
         if (rc) return rc;
     }
     HF_CHECK(cudaMemsetAsync(h->d_G, 0, (size_t)h->nb * h->nb * sizeof(double), h->stream));
-    int rc = launch_diag(h, 0, p_dev, thr);
+    int rc = fork_diag(h, 0, p_dev, thr, true);
     if (rc) return rc;
     if ((rc = launch_symm(h, f_dev))) return rc;
     return build_active(h);  // reads the Schwarz factors back (synchronises the handle's stream)
@@ -1716,6 +1819,6 @@ extern "C" int hfgpu_fock_build_diag_static(hfgpu_handle* h, double* f_dev, cons
     // G keeps the previous call's sums: clear it first
     HF_CHECK(cudaMemsetAsync(G, 0, (size_t)h->nb * h->nb * sizeof(double), h->stream));
     if ((rc = launch_maxdm(h, p_dev, md))) return rc;
-    if ((rc = launch_diag(h, 1, p_dev, thr, G, md))) return rc;
+    if ((rc = launch_diag(h, 1, p_dev, thr, G, md, h->stream, h->stream))) return rc;
     return launch_symm(h, f_dev, G);
 }

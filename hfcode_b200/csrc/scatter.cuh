@@ -1,95 +1,85 @@
-// J/K scatter of one shell quartet's ERI block held in memory with a stride
-// (the staged classes' scratch), into the one-triangle buffer G
-// (F += G + G^T later), one FP64 atomic per block element:
+// J/K scatter of one shell quartet's ERI block, shared by `nl` lanes, into
+// the one-triangle buffer G (F += G + G^T later), one FP64 atomic per block
+// element:
 //   J_ab += 2s P_cd e,  J_cd += 2s P_ab e,
 //   K_ac -= s/2 P_bd e, K_ad -= s/2 P_bc e, K_bc -= s/2 P_ad e, K_bd -= s/2 P_ac e.
-// One pass over the block: the first index i is a loop, (j, k, l) are
-// unrolled, so every element is read once; blocks indexed by i are flushed
-// per i, the others once at the end.  Host-compilable with the shims of the
-// test harness.
+// The quartet's density blocks go to `w` first; then lane x, x + nl, ... of
+// the block elements (16 to 25 per block) each sum their row of products.
+// With one thread per quartet the (dd|dd) block is a serial chain of 625
+// element loads and 3750 FMAs, which a small molecule has nothing to hide
+// behind: 288 us for the 21 (dd|dd) diagonal quartets of benzene.
+// Host-compilable with the shims of the test harness (lane 0 of 1).
 #pragma once
 #include "types.cuh"
 
 namespace hfgpu {
 
-template <int NA, int NB, int NC, int ND>
-__device__ __forceinline__ void scatter_strided(const double* __restrict__ e, size_t st, double s,
-                                                const GPair& bra, const GPair& ket,
-                                                const double* __restrict__ P, double* __restrict__ G, int nb,
-                                                bool jonly) {
+// Density elements a quartet's scatter reads: P_cd, P_ab, P_bd, P_bc, P_ad, P_ac.
+__host__ __device__ constexpr int scatter_dens(int NA, int NB, int NC, int ND) {
+    return NC * ND + NA * NB + NB * ND + NB * NC + NA * ND + NA * NC;
+}
+
+template <int NA, int NB, int NC, int ND, typename E>
+__device__ __forceinline__ void scatter_lanes(const E* e, double* w, double s, const GPair& bra, const GPair& ket,
+                                              const double* __restrict__ P, double* __restrict__ G, int nb,
+                                              bool jonly, int lane, int nl) {
     const int a0 = bra.aoa, b0 = bra.aob, c0 = ket.aoa, d0 = ket.aob;
-    auto Pm = [&](int r, int c) { return __ldg(P + r + (size_t)c * nb); };
-    auto Ga = [&](int r, int c) { return G + r + (size_t)c * nb; };
-    const double s2 = 2.0 * s, hs = -0.5 * s;
-    double jcd[NC * ND], kbc[NB * NC], kbd[NB * ND], pcd[NC * ND];
-#pragma unroll
-    for (int x = 0; x < NC * ND; ++x) jcd[x] = 0.0;
-#pragma unroll
-    for (int x = 0; x < NB * NC; ++x) kbc[x] = 0.0;
-#pragma unroll
-    for (int x = 0; x < NB * ND; ++x) kbd[x] = 0.0;
-#pragma unroll
-    for (int k = 0; k < NC; ++k)
-#pragma unroll
-        for (int l = 0; l < ND; ++l) pcd[k * ND + l] = Pm(c0 + k, d0 + l);
-#pragma unroll 1
-    for (int i = 0; i < NA; ++i) {
-        double jab[NB], kac[NC], kad[ND], pad_[ND], pac[NC];
-#pragma unroll
-        for (int j = 0; j < NB; ++j) jab[j] = 0.0;
-#pragma unroll
-        for (int k = 0; k < NC; ++k) {
-            kac[k] = 0.0;
-            pac[k] = Pm(a0 + i, c0 + k);
-        }
-#pragma unroll
-        for (int l = 0; l < ND; ++l) {
-            kad[l] = 0.0;
-            pad_[l] = Pm(a0 + i, d0 + l);
-        }
-        const double* ei = e + (size_t)(i * NB * NC * ND) * st;
-#pragma unroll
-        for (int j = 0; j < NB; ++j) {
-            const double pab = Pm(a0 + i, b0 + j);
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                const double pbc = Pm(b0 + j, c0 + k);
-#pragma unroll
-                for (int l = 0; l < ND; ++l) {
-                    const double v = __ldg(ei + (size_t)((j * NC + k) * ND + l) * st);
-                    jab[j] += pcd[k * ND + l] * v;
-                    jcd[k * ND + l] += pab * v;
-                    if (!jonly) {
-                        kac[k] += Pm(b0 + j, d0 + l) * v;
-                        kad[l] += pbc * v;
-                        kbc[j * NC + k] += pad_[l] * v;
-                        kbd[j * ND + l] += pac[k] * v;
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < NB; ++j) atomicAdd(Ga(a0 + i, b0 + j), s2 * jab[j]);
-        if (!jonly) {
-#pragma unroll
-            for (int k = 0; k < NC; ++k) atomicAdd(Ga(a0 + i, c0 + k), hs * kac[k]);
-#pragma unroll
-            for (int l = 0; l < ND; ++l) atomicAdd(Ga(a0 + i, d0 + l), hs * kad[l]);
-        }
+    double *pcd = w, *pab = pcd + NC * ND, *pbd = pab + NA * NB, *pbc = pbd + NB * ND, *pad_ = pbc + NB * NC,
+           *pac = pad_ + NA * ND;
+    // block (r, c) of P, row-major; P is symmetric and column-major
+    auto fetch = [&](double* dst, int r0, int nr, int cc0, int nc) {
+        for (int x = lane; x < nr * nc; x += nl) dst[x] = __ldg(P + (cc0 + x % nc) + (size_t)(r0 + x / nc) * nb);
+    };
+    fetch(pcd, c0, NC, d0, ND);
+    fetch(pab, a0, NA, b0, NB);
+    if (!jonly) {
+        fetch(pbd, b0, NB, d0, ND);
+        fetch(pbc, b0, NB, c0, NC);
+        fetch(pad_, a0, NA, d0, ND);
+        fetch(pac, a0, NA, c0, NC);
     }
-#pragma unroll
-    for (int k = 0; k < NC; ++k)
-#pragma unroll
-        for (int l = 0; l < ND; ++l) atomicAdd(Ga(c0 + k, d0 + l), s2 * jcd[k * ND + l]);
-    if (jonly) return;
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-#pragma unroll
-        for (int k = 0; k < NC; ++k) atomicAdd(Ga(b0 + j, c0 + k), hs * kbc[j * NC + k]);
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-#pragma unroll
-        for (int l = 0; l < ND; ++l) atomicAdd(Ga(b0 + j, d0 + l), hs * kbd[j * ND + l]);
+#ifdef __CUDA_ARCH__
+    __syncwarp();
+#endif
+    constexpr int SI = NB * NC * ND, SJ = NC * ND, SK = ND;  // strides of i, j, k in the block
+    constexpr int O1 = NA * NB, O2 = O1 + NC * ND, O3 = O2 + NA * NC, O4 = O3 + NA * ND, O5 = O4 + NB * NC,
+                  O6 = O5 + NB * ND;
+    const int nel = jonly ? O2 : O6;
+    for (int x = lane; x < nel; x += nl) {
+        // element (r, c) of its block: first product, two loops over the others
+        int y, r, c, base, n1, s1, n2, s2;
+        const double* d;
+        double* g;
+        if (x < O1) {
+            y = x, r = y / NB, c = y % NB;
+            base = r * SI + c * SJ, n1 = NC, s1 = SK, n2 = ND, s2 = 1, d = pcd;
+            g = G + (a0 + r) + (size_t)(b0 + c) * nb;
+        } else if (x < O2) {
+            y = x - O1, r = y / ND, c = y % ND;
+            base = r * SK + c, n1 = NA, s1 = SI, n2 = NB, s2 = SJ, d = pab;
+            g = G + (c0 + r) + (size_t)(d0 + c) * nb;
+        } else if (x < O3) {
+            y = x - O2, r = y / NC, c = y % NC;
+            base = r * SI + c * SK, n1 = NB, s1 = SJ, n2 = ND, s2 = 1, d = pbd;
+            g = G + (a0 + r) + (size_t)(c0 + c) * nb;
+        } else if (x < O4) {
+            y = x - O3, r = y / ND, c = y % ND;
+            base = r * SI + c, n1 = NB, s1 = SJ, n2 = NC, s2 = SK, d = pbc;
+            g = G + (a0 + r) + (size_t)(d0 + c) * nb;
+        } else if (x < O5) {
+            y = x - O4, r = y / NC, c = y % NC;
+            base = r * SJ + c * SK, n1 = NA, s1 = SI, n2 = ND, s2 = 1, d = pad_;
+            g = G + (b0 + r) + (size_t)(c0 + c) * nb;
+        } else {
+            y = x - O5, r = y / ND, c = y % ND;
+            base = r * SJ + c, n1 = NA, s1 = SI, n2 = NC, s2 = SK, d = pac;
+            g = G + (b0 + r) + (size_t)(d0 + c) * nb;
+        }
+        double acc = 0.0;
+        for (int u = 0; u < n1; ++u)
+            for (int v = 0; v < n2; ++v) acc += d[u * n2 + v] * (double)e[base + u * s1 + v * s2];
+        atomicAdd(g, (x < O2 ? 2.0 * s : -0.5 * s) * acc);
+    }
 }
 
 }  // namespace hfgpu

@@ -86,6 +86,26 @@ __device__ __forceinline__ GPrim load_prim(const PrimSoA& s, int i) {
     return g;
 }
 
+// The share of a quartet's primitive loops that one thread runs: bra
+// primitives ib, ib + db, ..., ket primitives ik, ik + dk, ...; `n`
+// consecutive lanes of a warp share the quartet and sum its contracted
+// accumulators.  {0, 1, 0, 1, 1} is one thread per quartet.
+struct LaneSplit {
+    int ib, db, ik, dk, n;
+};
+
+__device__ __forceinline__ constexpr LaneSplit one_lane() { return LaneSplit{0, 1, 0, 1, 1}; }
+
+// Butterfly step of the sum over a quartet's lanes (all lanes of the warp call it).
+template <typename T>
+__device__ __forceinline__ T lane_add(T x, int o) {
+#ifdef __CUDA_ARCH__
+    return x + __shfl_xor_sync(0xffffffffu, x, o);
+#else
+    return x;
+#endif
+}
+
 // ---------------------------------------------------------------- Boys ----
 // F_m(T) for m = 0..M.  T > 28: F_0 = sqrt(pi/T)/2 and upward recursion
 // without the exponential, which is what the reference evaluates there
