@@ -35,124 +35,150 @@ __host__ __device__ constexpr int pt_nb(int t) {
         }                                                                                            \
     };
 
-// ------------------------------------------------------------ scatter ----
-// F contributions of one shell quartet with uniform weight s, into the
-// one-triangle buffer G (F += G + G^T later).  Column-major P(r,c)=P[r+c*nb].
-template <int NA, int NB, int NC, int ND, typename E>
-__device__ __forceinline__ void scatter_quartet(const E* e, double s, int a0, int b0, int c0, int d0,
-                                                const double* __restrict__ P, double* __restrict__ G,
-                                                int nb, bool jonly) {
-    auto Pm = [&](int r, int c) { return __ldg(P + r + (size_t)c * nb); };
-    auto idx = [](int i, int j, int k, int l) { return ((i * NB + j) * NC + k) * ND + l; };
-    double pcd[NC * ND], pab[NA * NB];
+// ------------------------------------------------------- warp output ----
+// The J/K sums of a warp's 32 quartets go into G element by element across
+// the lanes: the lanes write their quartets' sums of up to N elements to a
+// shared buffer ([element][quartet], WST apart), then lane v owns element v
+// and walks the quartets, adding up the runs of quartets that share the block
+// (consecutive entries of a list mostly share the bra pair and the ket's
+// first shell) with one atomic per run.  The lanes of one atomic instruction
+// then lie in one or two blocks of G, which are contiguous: a warp's atomics
+// touch 2-3 cache lines instead of 32.  With one atomic per element and lane
+// the L1 tag stage (one line per cycle) bounded every scatter: 110 atomic
+// instructions of 31 lines per warp for LL|DL, l1tex throughput 55-62% in
+// all scatter kernels while the FP64 pipe idled.
+constexpr int WST = 33;  // odd stride: a column is written and read without bank conflicts
+
+// Block offsets of the warp's quartets in G: [block type][quartet], in the
+// order of Blocks (ab, cd, ac, ad, bc, bd); -1 for lanes without a quartet.
+constexpr int NBASE = 6 * WST;
+__device__ __forceinline__ void set_bases(int* base, const int* __restrict__ boff, int nsh, const GPair& bra,
+                                          const GPair& ket, bool act) {
+    const int lane = threadIdx.x & 31;
+    const int s[6][2] = {{bra.sa, bra.sb}, {ket.sa, ket.sb}, {bra.sa, ket.sa},
+                         {bra.sa, ket.sb}, {bra.sb, ket.sa}, {bra.sb, ket.sb}};
 #pragma unroll
-    for (int k = 0; k < NC; ++k)
-#pragma unroll
-        for (int l = 0; l < ND; ++l) pcd[k * ND + l] = Pm(c0 + k, d0 + l);
-#pragma unroll
-    for (int i = 0; i < NA; ++i)
-#pragma unroll
-        for (int j = 0; j < NB; ++j) pab[i * NB + j] = Pm(a0 + i, b0 + j);
-    const double s2 = 2.0 * s;
-    // J_ab and J_cd
-#pragma unroll
-    for (int i = 0; i < NA; ++i)
-#pragma unroll
-        for (int j = 0; j < NB; ++j) {
-            double acc = 0.0;
-#pragma unroll
-            for (int k = 0; k < NC; ++k)
-#pragma unroll
-                for (int l = 0; l < ND; ++l) acc += pcd[k * ND + l] * (double)e[idx(i, j, k, l)];
-            atomicAdd(G + (a0 + i) + (size_t)(b0 + j) * nb, s2 * acc);
+    for (int x = 0; x < 6; ++x) base[x * WST + lane] = act ? __ldg(boff + s[x][0] * nsh + s[x][1]) : -1;
+}
+
+// Adds elements [0, n) of the buffer (n <= N, warp-uniform): map(v, type, off)
+// gives element v's block type and place in the block.  N <= 16 lets two, N
+// <= 8 four groups of lanes walk a half or a quarter of the quartets each.
+// The caller synchronises the warp before (the buffer is written) and after.
+template <int N, typename E, typename Map>
+__device__ __forceinline__ void walk_add(const E* tb, const int* base, int n, double* __restrict__ G, Map map) {
+    constexpr int NG = N <= 8 ? 4 : N <= 16 ? 2 : 1, W = 32 / NG;  // groups; lanes (and quartets) per group
+    const int lane = threadIdx.x & 31, q0 = lane / W * W;
+#pragma unroll 1
+    for (int v = lane % W; v < n; v += W) {
+        int type, off;
+        map(v, type, off);
+        const int* b = base + type * WST + q0;
+        const E* t = tb + v * WST + q0;
+        double sum = 0.0;
+        int cur = -1;
+#pragma unroll 4
+        for (int q = 0; q < W; ++q) {
+            const int x = b[q];
+            if (x != cur) {
+                if (cur >= 0) atomicAdd(G + cur + off, sum);
+                cur = x;
+                sum = 0.0;
+            }
+            sum += (double)t[q];
         }
-#pragma unroll
-    for (int k = 0; k < NC; ++k)
-#pragma unroll
-        for (int l = 0; l < ND; ++l) {
-            double acc = 0.0;
-#pragma unroll
-            for (int i = 0; i < NA; ++i)
-#pragma unroll
-                for (int j = 0; j < NB; ++j) acc += pab[i * NB + j] * (double)e[idx(i, j, k, l)];
-            atomicAdd(G + (c0 + k) + (size_t)(d0 + l) * nb, s2 * acc);
-        }
-    if (jonly) return;
-    const double hs = -0.5 * s;
-    // K_ac (sum over j,l of P_jl), K_ad (P_jk), K_bc (P_il), K_bd (P_ik)
-    {
-        double pbd[NB * ND];
-#pragma unroll
-        for (int j = 0; j < NB; ++j)
-#pragma unroll
-            for (int l = 0; l < ND; ++l) pbd[j * ND + l] = Pm(b0 + j, d0 + l);
-#pragma unroll
-        for (int i = 0; i < NA; ++i)
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                double acc = 0.0;
-#pragma unroll
-                for (int j = 0; j < NB; ++j)
-#pragma unroll
-                    for (int l = 0; l < ND; ++l) acc += pbd[j * ND + l] * (double)e[idx(i, j, k, l)];
-                atomicAdd(G + (a0 + i) + (size_t)(c0 + k) * nb, hs * acc);
-            }
-    }
-    {
-        double pbc[NB * NC];
-#pragma unroll
-        for (int j = 0; j < NB; ++j)
-#pragma unroll
-            for (int k = 0; k < NC; ++k) pbc[j * NC + k] = Pm(b0 + j, c0 + k);
-#pragma unroll
-        for (int i = 0; i < NA; ++i)
-#pragma unroll
-            for (int l = 0; l < ND; ++l) {
-                double acc = 0.0;
-#pragma unroll
-                for (int j = 0; j < NB; ++j)
-#pragma unroll
-                    for (int k = 0; k < NC; ++k) acc += pbc[j * NC + k] * (double)e[idx(i, j, k, l)];
-                atomicAdd(G + (a0 + i) + (size_t)(d0 + l) * nb, hs * acc);
-            }
-    }
-    {
-        double pad_[NA * ND];
-#pragma unroll
-        for (int i = 0; i < NA; ++i)
-#pragma unroll
-            for (int l = 0; l < ND; ++l) pad_[i * ND + l] = Pm(a0 + i, d0 + l);
-#pragma unroll
-        for (int j = 0; j < NB; ++j)
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                double acc = 0.0;
-#pragma unroll
-                for (int i = 0; i < NA; ++i)
-#pragma unroll
-                    for (int l = 0; l < ND; ++l) acc += pad_[i * ND + l] * (double)e[idx(i, j, k, l)];
-                atomicAdd(G + (b0 + j) + (size_t)(c0 + k) * nb, hs * acc);
-            }
-    }
-    {
-        double pac[NA * NC];
-#pragma unroll
-        for (int i = 0; i < NA; ++i)
-#pragma unroll
-            for (int k = 0; k < NC; ++k) pac[i * NC + k] = Pm(a0 + i, c0 + k);
-#pragma unroll
-        for (int j = 0; j < NB; ++j)
-#pragma unroll
-            for (int l = 0; l < ND; ++l) {
-                double acc = 0.0;
-#pragma unroll
-                for (int i = 0; i < NA; ++i)
-#pragma unroll
-                    for (int k = 0; k < NC; ++k) acc += pac[i * NC + k] * (double)e[idx(i, j, k, l)];
-                atomicAdd(G + (b0 + j) + (size_t)(d0 + l) * nb, hs * acc);
-            }
+        if (cur >= 0) atomicAdd(G + cur + off, sum);
     }
 }
+
+// ------------------------------------------------------------ scatter ----
+// F contributions of the 32 quartets of a warp, blocks in registers (direct
+// classes), with weight s, into the one-triangle buffer G (F += G + G^T
+// later).  P and G are in shell-pair blocks.  `tb` and `base`: the warp's
+// shared buffers.  Every lane of the warp calls it; those with act false add
+// nothing.
+constexpr int DCH = 16;  // elements per pass through the buffer
+template <int NA, int NB, int NC, int ND, typename E>
+__device__ __forceinline__ void scatter_quartet(const E* e, double s, const GPair& bra, const GPair& ket, bool act,
+                                                const double* __restrict__ Pb, const int* __restrict__ boff, int nsh,
+                                                double* __restrict__ G, bool jonly, double* tb, int* base) {
+    using X = Blocks<NA, NB, NC, ND>;
+    const int lane = threadIdx.x & 31;
+    const double* __restrict__ Pab = Pb + __ldg(boff + bra.sa * nsh + bra.sb);
+    const double* __restrict__ Pcd = Pb + __ldg(boff + ket.sa * nsh + ket.sb);
+    const double* __restrict__ Pac = Pb + __ldg(boff + bra.sa * nsh + ket.sa);
+    const double* __restrict__ Pad = Pb + __ldg(boff + bra.sa * nsh + ket.sb);
+    const double* __restrict__ Pbc = Pb + __ldg(boff + bra.sb * nsh + ket.sa);
+    const double* __restrict__ Pbd = Pb + __ldg(boff + bra.sb * nsh + ket.sb);
+    __syncwarp();  // the previous pass has been read
+    set_bases(base, boff, nsh, bra, ket, act);
+    const double s2 = 2.0 * s, hs = -0.5 * s;
+    auto E4 = [&](int i, int j, int k, int l) { return (double)e[((i * NB + j) * NC + k) * ND + l]; };
+    const int nel = jonly ? X::AC : X::END;
+#pragma unroll
+    for (int c = 0; c < X::END; c += DCH) {
+        if (c >= nel) break;
+        if (c > 0) __syncwarp();  // the previous chunk has been read
+#pragma unroll
+        for (int x = c; x < (c + DCH < X::END ? c + DCH : X::END); ++x) {
+            double acc = 0.0;
+            if (x < X::CD) {
+#pragma unroll
+                for (int k = 0; k < NC; ++k)
+#pragma unroll
+                    for (int l = 0; l < ND; ++l) acc += __ldg(Pcd + k * ND + l) * E4(x / NB, x % NB, k, l);
+            } else if (x < X::AC) {
+                const int y = x - X::CD;
+#pragma unroll
+                for (int i = 0; i < NA; ++i)
+#pragma unroll
+                    for (int j = 0; j < NB; ++j) acc += __ldg(Pab + i * NB + j) * E4(i, j, y / ND, y % ND);
+            } else if (x < X::AD) {
+                const int y = x - X::AC;
+#pragma unroll
+                for (int j = 0; j < NB; ++j)
+#pragma unroll
+                    for (int l = 0; l < ND; ++l) acc += __ldg(Pbd + j * ND + l) * E4(y / NC, j, y % NC, l);
+            } else if (x < X::BC) {
+                const int y = x - X::AD;
+#pragma unroll
+                for (int j = 0; j < NB; ++j)
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) acc += __ldg(Pbc + j * NC + k) * E4(y / ND, j, k, y % ND);
+            } else if (x < X::BD) {
+                const int y = x - X::BC;
+#pragma unroll
+                for (int i = 0; i < NA; ++i)
+#pragma unroll
+                    for (int l = 0; l < ND; ++l) acc += __ldg(Pad + i * ND + l) * E4(i, y / NC, y % NC, l);
+            } else {
+                const int y = x - X::BD;
+#pragma unroll
+                for (int i = 0; i < NA; ++i)
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) acc += __ldg(Pac + i * NC + k) * E4(i, y / ND, k, y % ND);
+            }
+            tb[(x - c) * WST + lane] = (x < X::AC ? s2 : hs) * acc;
+        }
+        __syncwarp();
+        walk_add<DCH>(tb, base, min(DCH, nel - c), G, [&](int v, int& type, int& off) {
+            const int x = c + v;
+            type = x < X::CD ? 0 : x < X::AC ? 1 : x < X::AD ? 2 : x < X::BC ? 3 : x < X::BD ? 4 : 5;
+            off = x - (x < X::CD ? 0 : x < X::AC ? X::CD : x < X::AD ? X::AC : x < X::BC ? X::AD
+                       : x < X::BD ? X::BC : X::BD);
+        });
+    }
+}
+
+// Elements of G (shell-pair blocks) for scatter_lanes.
+struct BlockDst {
+    double* G;
+    const int* boff;
+    int nsh;
+    __device__ __forceinline__ double* operator()(int s1, int s2, int, int, int y) const {
+        return G + __ldg(boff + s1 * nsh + s2) + y;
+    }
+};
 
 // ------------------------------------------------------- kernel args ----
 struct ClassStats {
@@ -232,9 +258,10 @@ struct NDArgs {
     PrimSoA prims;
     const double* boys;     // global table, [M][225][8]
     const float* boysf;
-    const double* P;
-    double* G;
-    int nb;
+    const double* Pb;       // density in shell-pair blocks
+    double* G;              // in shell-pair blocks
+    const int* boff;        // block offsets, nsh x nsh
+    int nsh;
     double thr;
     int jonly;
     ClassStats* stats;
@@ -284,8 +311,10 @@ __global__ void __launch_bounds__(ND_THREADS) k_nondiag(NDArgs a) {
     else stage_boys<C::LL>(sboys, a.boys);
     constexpr int NA = pt_na(C::BI), NB = pt_nb(C::BI), NC = pt_na(C::KI), ND = pt_nb(C::KI);
     static_assert(NA * NB * NC * ND == C::NOUT, "class size");
+    __shared__ double tbuf[ND_THREADS / 32][DCH * WST];
+    __shared__ int tbase[ND_THREADS / 32][NBASE];
     unsigned long long nsc = 0, npr = 0;
-    const int warps = gridDim.x * (ND_THREADS / 32);
+    const int warps = gridDim.x * (ND_THREADS / 32), wp = threadIdx.x >> 5;
     Unit w;
     for (int u = u0 + (threadIdx.x >> 5); unit_of(a.list, u, w); u += warps) {
         const GPair bra = a.bra[w.q.x];
@@ -293,15 +322,15 @@ __global__ void __launch_bounds__(ND_THREADS) k_nondiag(NDArgs a) {
         Real e[C::NOUT];
         if constexpr (F32) C::eri32(bra, ket, a.prims, sboys, w.ls, e);
         else C::eri(bra, ket, a.prims, sboys, w.ls, e);
-        if (!w.store) continue;
-        npr += (unsigned long long)(bra.np * ket.np);
         Real mx = 0;
 #pragma unroll
         for (int i = 0; i < C::NOUT; ++i) mx = fmax(mx, fabs(e[i]));
-        if ((double)mx < a.thr) continue;  // fock_build_non_diag.f90:69
-        ++nsc;
+        const bool act = w.store && !((double)mx < a.thr);  // fock_build_non_diag.f90:69
+        npr += w.store ? (unsigned long long)(bra.np * ket.np) : 0ull;
+        nsc += act ? 1ull : 0ull;
         const double s = (bra.sa == bra.sb ? 0.5 : 1.0) * (ket.sa == ket.sb ? 0.5 : 1.0);
-        scatter_quartet<NA, NB, NC, ND>(e, s, bra.aoa, bra.aob, ket.aoa, ket.aob, a.P, a.G, a.nb, a.jonly);
+        scatter_quartet<NA, NB, NC, ND>(e, s, bra, ket, act, a.Pb, a.boff, a.nsh, a.G, a.jonly != 0, tbuf[wp],
+                                        tbase[wp]);
     }
     if (a.stats) warp_add_stats(a.stats, nsc, npr, F32 ? nsc : 0ull);
 }
@@ -315,7 +344,8 @@ struct DiagArgs {
     const double* md;      // mode 1: nsh x nsh maxdm
     int nsh;
     const double* P;
-    double* G;
+    double* G;             // in shell-pair blocks
+    const int* boff;       // block offsets, nsh x nsh
     int nb;
     double thr;
 };
@@ -337,20 +367,23 @@ __global__ void __launch_bounds__(ND_THREADS) k_diag(DiagArgs a) {
     if (t >= a.n) return;
     const GPair pr = a.pairs[t];
     if (MODE == 1 && diag_screened(pr, a.schw[t], a.md, a.nsh, a.thr)) return;
+    __shared__ double sw[ND_THREADS / 32][scatter_dens(NA, NB, NA, NB)], se[ND_THREADS / 32][C::NOUT];
+    const int wp = threadIdx.x >> 5;
     double e[C::NOUT];
     C::eri(pr, pr, a.prims, a.boys + (size_t)C::LL * BOYS_BLK, LaneSplit{lane >> 3, 4, lane & 7, 8, 32}, e);
-    if (lane) return;
     if (MODE == 0) {
         double mx = 0;
 #pragma unroll
         for (int i = 0; i < C::NOUT; ++i) mx = fmax(mx, fabs(e[i]));
-        a.schw[t] = sqrt(mx);
+        if (lane == 0) a.schw[t] = sqrt(mx);
     }
+    if (lane == 0) {
 #pragma unroll
-    for (int i = 0; i < C::NOUT; ++i)
-        if (!(fabs(e[i]) > INTTHRESH)) e[i] = 0.0;  // element skip
+        for (int i = 0; i < C::NOUT; ++i) se[wp][i] = fabs(e[i]) > INTTHRESH ? e[i] : 0.0;  // element skip
+    }
     const double f = pr.sa == pr.sb ? 1.0 : 2.0;
-    scatter_quartet<NA, NB, NA, NB>(e, f * f / 8.0, pr.aoa, pr.aob, pr.aoa, pr.aob, a.P, a.G, a.nb, false);
+    scatter_lanes<NA, NB, NA, NB>(se[wp], sw[wp], f * f / 8.0, pr, pr, a.P, a.nb, BlockDst{a.G, a.boff, a.nsh}, false,
+                                  lane, 32);
 }
 
 
@@ -462,13 +495,23 @@ __device__ __forceinline__ void cp_async_elem(E* dst, const E* src) {
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(src) : "memory");
 }
 
-// Shared-memory plan of the async scatter (element size es): three slab
-// buffers when they fit two blocks per SM, else two.
+// Shared-memory plan of the async scatter (element size es), per warp: NBUF
+// slab buffers (three when they fit two blocks per SM, else two), P_bc and
+// P_bd, the output buffer of one i (in the slab just consumed where that is
+// large enough) and the block offsets.  The last output pass, J_cd, K_bc and
+// K_bd, goes through the slab buffers and the P rows, which are free then.
+__host__ __device__ constexpr bool scat_over(int NB, int NC, int ND) { return NC * ND * 32 >= (NB + NC + ND) * WST; }
+__host__ __device__ constexpr int scat_warp_elems(int nbuf, int NB, int NC, int ND) {
+    return (nbuf * NC * ND + NB * (NC + ND)) * 32 + (scat_over(NB, NC, ND) ? 0 : (NB + NC + ND) * WST);
+}
+__host__ __device__ constexpr int scat_bytes(int nbuf, int NB, int NC, int ND, int es) {
+    return (ND_THREADS / 32) * (scat_warp_elems(nbuf, NB, NC, ND) * es + NBASE * 4);
+}
 __host__ __device__ constexpr int scat_nbuf(int NA, int NB, int NC, int ND, int es = 8) {
-    return (3 * NC * ND + NB * (NC + ND)) * ND_THREADS * es <= 110 * 1024 ? 3 : 2;
+    return scat_bytes(3, NB, NC, ND, es) <= 112 * 1024 ? 3 : 2;
 }
 __host__ __device__ constexpr int scat_smem_bytes(int NA, int NB, int NC, int ND, int es = 8) {
-    return (scat_nbuf(NA, NB, NC, ND, es) * NC * ND + NB * (NC + ND)) * ND_THREADS * es;
+    return scat_bytes(scat_nbuf(NA, NB, NC, ND, es), NB, NC, ND, es);
 }
 
 // E is the element type of the scratch rows and of the block sums: double
@@ -478,11 +521,16 @@ template <int NA, int NB, int NC, int ND, typename E>
 __device__ __forceinline__ void scatter_async(const E* __restrict__ e, size_t st, double s, const GPair& bra,
                                               const GPair& ket, const double* __restrict__ Pb,
                                               const int* __restrict__ boff, int nsh,
-                                              double* __restrict__ G, int nb, bool jonly, bool act, E* sm) {
-    constexpr int T = ND_THREADS, SLAB = NC * ND, NS = NA * NB;
+                                              double* __restrict__ G, bool jonly, bool act, char* smem) {
+    constexpr int SLAB = NC * ND, NS = NA * NB;
     constexpr int NBUF = scat_nbuf(NA, NB, NC, ND, (int)sizeof(E));
-    const int tid = threadIdx.x;
-    const int a0 = bra.aoa, b0 = bra.aob, c0 = ket.aoa, d0 = ket.aob;
+    constexpr int NI = NB + NC + ND;                 // outputs of one i: J_ab, K_ac, K_ad
+    constexpr int NF = NC * ND + NB * NC + NB * ND;  // and at the end: J_cd, K_bc, K_bd
+    static_assert((NBUF * SLAB + NB * (NC + ND)) * 32 >= NF * WST, "the last outputs fit the freed buffers");
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    char* mine = smem + wp * (scat_warp_elems(NBUF, NB, NC, ND) * (int)sizeof(E) + NBASE * 4);
+    E* wb = reinterpret_cast<E*>(mine + NBASE * 4);  // the warp's buffers
+    int* base = reinterpret_cast<int*>(mine);
     // density blocks in shell-pair order (row-major within a block), so each
     // row a thread reads is contiguous instead of one access per column
     const double* __restrict__ Bab = Pb + __ldg(boff + bra.sa * nsh + bra.sb);
@@ -491,46 +539,26 @@ __device__ __forceinline__ void scatter_async(const E* __restrict__ e, size_t st
     const double* __restrict__ Bbc = Pb + __ldg(boff + bra.sb * nsh + ket.sa);
     const double* __restrict__ Bbd = Pb + __ldg(boff + bra.sb * nsh + ket.sb);
     const double* __restrict__ Bcd = Pb + __ldg(boff + ket.sa * nsh + ket.sb);
-    auto Ga = [&](int r, int c) { return G + r + (size_t)c * nb; };
-    // The quartets of a warp are consecutive entries of a compacted list:
-    // they mostly share their bra pair, and the active lists are ordered by
-    // first shell within each primitive-count group, so they mostly share the
-    // ket's first shell too.  A block element whose row and column shells are
-    // the same in every lane has one address for the whole warp: its sums are
-    // reduced across the warp and added with one atomic.
-    const int lane = threadIdx.x & 31;
-    auto same = [](int x) { return __all_sync(0xffffffffu, x == __shfl_sync(0xffffffffu, x, 0)); };
-    const bool ua = same(a0), ub = same(b0), uc = same(c0), ud = same(d0);
-    const bool wuni = ua && ub;
-    // every lane calls this with the same `uni` (lanes without a quartet add 0)
-    auto emit = [&](double* addr, double v, bool uni) {
-        if (uni) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) atomicAdd(addr, v);
-        } else if (act) {
-            atomicAdd(addr, v);
-        }
-    };
-    E* eb = sm + tid;                      // [NBUF][SLAB][T], this thread's column
-    E* pk = sm + NBUF * SLAB * T + tid;    // [NB*NC] P_bc then [NB*ND] P_bd
+    E* eb = wb + lane;                       // [NBUF][SLAB][32], this lane's column
+    E* pk = wb + NBUF * SLAB * 32 + lane;    // [NB*NC] P_bc then [NB*ND] P_bd
     auto issue = [&](int slab) {
         if (slab < NS) {
             const E* src = e + (size_t)slab * SLAB * st;
-            E* dst = eb + (slab % NBUF) * SLAB * T;
+            E* dst = eb + (slab % NBUF) * SLAB * 32;
 #pragma unroll
-            for (int r = 0; r < SLAB; ++r) cp_async_elem(dst + r * T, src + (size_t)r * st);
+            for (int r = 0; r < SLAB; ++r) cp_async_elem(dst + r * 32, src + (size_t)r * st);
         }
         cp_async_commit();  // empty groups keep the count uniform
     };
 #pragma unroll
     for (int q = 0; q < NBUF - 1; ++q) issue(q);
+    set_bases(base, boff, nsh, bra, ket, act);
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
 #pragma unroll
-        for (int k = 0; k < NC; ++k) pk[(j * NC + k) * T] = (E)__ldg(Bbc + j * NC + k);
+        for (int k = 0; k < NC; ++k) pk[(j * NC + k) * 32] = (E)__ldg(Bbc + j * NC + k);
 #pragma unroll
-        for (int l = 0; l < ND; ++l) pk[(NB * NC + j * ND + l) * T] = (E)__ldg(Bbd + j * ND + l);
+        for (int l = 0; l < ND; ++l) pk[(NB * NC + j * ND + l) * 32] = (E)__ldg(Bbd + j * ND + l);
     }
     const E s2 = (E)(2.0 * s), hs = (E)(-0.5 * s);
     E jcd[NC * ND], kbc[NB * NC], kbd[NB * ND], pcd[NC * ND];
@@ -564,18 +592,18 @@ __device__ __forceinline__ void scatter_async(const E* __restrict__ e, size_t st
             const int slab = i * NB + j;
             issue(slab + NBUF - 1);
             cp_async_wait<NBUF - 1>();  // this thread's copies of `slab` have landed
-            const E* es = eb + (slab % NBUF) * SLAB * T;
+            const E* es = eb + (slab % NBUF) * SLAB * 32;
             const E pab = (E)__ldg(Bab + i * NB + j);
 #pragma unroll
             for (int k = 0; k < NC; ++k) {
-                const E pbc = pk[(j * NC + k) * T];
+                const E pbc = pk[(j * NC + k) * 32];
 #pragma unroll
                 for (int l = 0; l < ND; ++l) {
-                    const E v = es[(k * ND + l) * T];
+                    const E v = es[(k * ND + l) * 32];
                     jab[j] += pcd[k * ND + l] * v;
                     jcd[k * ND + l] += pab * v;
                     if (!jonly) {
-                        kac[k] += pk[(NB * NC + j * ND + l) * T] * v;
+                        kac[k] += pk[(NB * NC + j * ND + l) * 32] * v;
                         kad[l] += pbc * v;
                         kbc[j * NC + k] += pad_[l] * v;
                         kbd[j * ND + l] += pac[k] * v;
@@ -583,32 +611,37 @@ __device__ __forceinline__ void scatter_async(const E* __restrict__ e, size_t st
                 }
             }
         }
+        // the outputs of this i through the slab just consumed (its next
+        // copies are issued in the next iteration) or their own buffer
+        E* tb = scat_over(NB, NC, ND) ? wb + (i * NB + NB - 1) % NBUF * SLAB * 32
+                                      : wb + (NBUF * SLAB + NB * (NC + ND)) * 32;
+        __syncwarp();
 #pragma unroll
-        for (int j = 0; j < NB; ++j) emit(Ga(a0 + i, b0 + j), act ? (double)(s2 * jab[j]) : 0.0, wuni);
-        if (!jonly) {
+        for (int j = 0; j < NB; ++j) tb[j * WST + lane] = s2 * jab[j];
 #pragma unroll
-            for (int k = 0; k < NC; ++k) emit(Ga(a0 + i, c0 + k), act ? (double)(hs * kac[k]) : 0.0, ua && uc);
+        for (int k = 0; k < NC; ++k) tb[(NB + k) * WST + lane] = hs * kac[k];
 #pragma unroll
-            for (int l = 0; l < ND; ++l) emit(Ga(a0 + i, d0 + l), act ? (double)(hs * kad[l]) : 0.0, ua && ud);
-        }
+        for (int l = 0; l < ND; ++l) tb[(NB + NC + l) * WST + lane] = hs * kad[l];
+        __syncwarp();
+        walk_add<NI>(tb, base, jonly ? NB : NI, G, [&](int v, int& type, int& off) {
+            type = v < NB ? 0 : v < NB + NC ? 2 : 3;
+            off = v < NB ? i * NB + v : v < NB + NC ? i * NC + v - NB : i * ND + v - NB - NC;
+        });
+        __syncwarp();
     }
     cp_async_wait<0>();
+    __syncwarp();
 #pragma unroll
-    for (int k = 0; k < NC; ++k)
+    for (int x = 0; x < NC * ND; ++x) wb[x * WST + lane] = s2 * jcd[x];
 #pragma unroll
-        for (int l = 0; l < ND; ++l)
-            emit(Ga(c0 + k, d0 + l), act ? (double)(s2 * jcd[k * ND + l]) : 0.0, uc && ud);
-    if (jonly) return;
+    for (int x = 0; x < NB * NC; ++x) wb[(NC * ND + x) * WST + lane] = hs * kbc[x];
 #pragma unroll
-    for (int j = 0; j < NB; ++j)
-#pragma unroll
-        for (int k = 0; k < NC; ++k)
-            emit(Ga(b0 + j, c0 + k), act ? (double)(hs * kbc[j * NC + k]) : 0.0, ub && uc);
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-#pragma unroll
-        for (int l = 0; l < ND; ++l)
-            emit(Ga(b0 + j, d0 + l), act ? (double)(hs * kbd[j * ND + l]) : 0.0, ub && ud);
+    for (int x = 0; x < NB * ND; ++x) wb[(NC * ND + NB * NC + x) * WST + lane] = hs * kbd[x];
+    __syncwarp();
+    walk_add<NF>(wb, base, jonly ? NC * ND : NF, G, [&](int v, int& type, int& off) {
+        type = v < NC * ND ? 1 : v < NC * ND + NB * NC ? 4 : 5;
+        off = v - (v < NC * ND ? 0 : v < NC * ND + NB * NC ? NC * ND : NC * ND + NB * NC);
+    });
 }
 
 // Post-screen (max |e| over all roles < thr, fock_build_non_diag.f90:69) and
@@ -638,218 +671,9 @@ __global__ void __launch_bounds__(ND_THREADS, sizeof(E) == 4 ? 3 : 2) k_scatter_
     const double s = (bra.sa == bra.sb ? 0.5 : 1.0) * (ket.sa == ket.sb ? 0.5 : 1.0);
     extern __shared__ __align__(16) double hf_scat_smem[];
     scatter_async<NA, NB, NC, ND, E>(reinterpret_cast<const E*>(a.out) + tcol(tq, NA * NB * NC * ND), TQ, s, bra,
-                                     ket, a.Pb, a.boff,
-                                     a.nsh, a.G, a.nb, a.jonly != 0, act, reinterpret_cast<E*>(hf_scat_smem));
+                                     ket, a.Pb, a.boff, a.nsh, a.G, a.jonly != 0, act,
+                                     reinterpret_cast<char*>(hf_scat_smem));
     if (a.stats) warp_add_stats(a.stats, nsc, npr, a.f32 ? nsc : 0ull);
-}
-
-// ------------------------------------- grouped staged scatter (4 lanes) ----
-// One quartet per group of SG = 4 lanes.  Lane g owns function g of one bra
-// shell O (S = 0: the first bra shell a, S = 1: the second, b), which has
-// four functions; X is the other bra shell.  The lane reads the rows of its
-// NX slabs (o = g, x = 0..NX-1), each NC*ND rows, and forms
-//   complete over the quartet:  J_OX[g][x] (P_cd), K_Oc[g][k] (P_Xd), K_Od[g][l] (P_Xc)
-//   summed over the group:      K_Xc[x][k] (P_Od), K_Xd[x][l] (P_Oc) after slab x,
-//                               J_cd[k][l] (P_OX) after the last slab
-// Group sums are two-step reduce-scatters (xor 1, xor 2), so each lane adds a
-// quarter of them and a quartet still issues one atomic per block element.
-// Against the one-thread scatter a thread holds about a third of the block
-// sums, which leaves room for more warps per SM to hide the latency of the
-// row and density loads.
-constexpr int SG = 4;
-__host__ __device__ constexpr int scatg_smem_bytes(int NX, int NC, int ND, int es) {
-    // two slab buffers of NC*ND rows per thread, then P_cd, P_Xc and P_Xd of
-    // each quartet of the block ([value][quartet])
-    return 2 * NC * ND * ND_THREADS * es + (NC * ND + NX * (NC + ND)) * (ND_THREADS / SG) * es;
-}
-// blocks per SM: as many as the shared memory allows, at most SCATG_BLK64
-// for FP64 sums and four for FP32 sums (128 registers)
-#ifndef SCATG_BLK64
-#define SCATG_BLK64 3
-#endif
-__host__ __device__ constexpr int scatg_cap(int es) { return es == 8 ? SCATG_BLK64 : 4; }
-__host__ __device__ constexpr int scatg_minb(int NX, int NC, int ND, int es) {
-    return 225 * 1024 / scatg_smem_bytes(NX, NC, ND, es) < scatg_cap(es) ? 225 * 1024 / scatg_smem_bytes(NX, NC, ND, es)
-                                                                         : scatg_cap(es);
-}
-
-// Sum N values over the four lanes of a group (reduce-scatter): on return
-// v[0 .. N/4) hold the group sums of elements base .. base + N/4 of the
-// input, base = (g&1 ? N/2 : 0) + (g&2 ? N/4 : 0).  N is a multiple of 4.
-template <int N, typename E>
-__device__ __forceinline__ int group_reduce_scatter(E* v, int g) {
-    constexpr int H1 = N / 2, H2 = N / 4;
-    const bool b0 = g & 1, b1 = g & 2;
-#pragma unroll
-    for (int i = 0; i < H1; ++i) {
-        const E lo = v[i], hi = v[H1 + i];
-        v[i] = (b0 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b0 ? lo : hi, 1);
-    }
-#pragma unroll
-    for (int i = 0; i < H2; ++i) {
-        const E lo = v[i], hi = v[H2 + i];
-        v[i] = (b1 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b1 ? lo : hi, 2);
-    }
-    return (b0 ? H1 : 0) + (b1 ? H2 : 0);
-}
-
-template <int NA, int NB, int NC, int ND, int S, typename E = double>
-__global__ void __launch_bounds__(ND_THREADS, scatg_minb(S == 0 ? NB : NA, NC, ND, (int)sizeof(E)))
-    k_scatter_grouped(StagedArgs a) {
-    constexpr int T = ND_THREADS, QB = T / SG, SLAB = NC * ND, NBUF = 2;
-    constexpr int NO = S == 0 ? NA : NB, NX = S == 0 ? NB : NA;
-    static_assert(NO == SG, "the lane-owned shell has four functions");
-    constexpr int NK = NC + ND, NK4 = (NK + 3) / 4 * 4;  // K_Xc[x], K_Xd[x] of one slab
-    constexpr int NJ4 = (NC * ND + 3) / 4 * 4;           // J_cd
-    constexpr int NPS = NC * ND + NX * NK;               // density values in shared memory
-    const int tid = threadIdx.x, lane = tid & 31, g = tid & (SG - 1), ql = tid / SG;
-    const int cnt = staged_count(a);
-    const int qi = blockIdx.x * QB + ql;
-    const int w0 = blockIdx.x * QB + (tid - lane) / SG;  // first quartet of this warp
-    if (w0 >= cnt) return;                              // whole warps only
-    // a group past the end works on the warp's first quartet and writes nothing
-    const bool valid = qi < cnt;
-    const int tq = valid ? qi : w0;
-    double mxq = 0.0;
-    const double* __restrict__ mxc = a.mx + tcol(tq, a.nroles);
-    for (int r = 0; r < a.nroles; ++r) mxq = fmax(mxq, mxc[r * TQ]);
-    const uint2 q = staged_quartet(a, tq);
-    const GPair bra = a.bra[q.x];
-    const GPair ket = a.ket[q.y];
-    const bool act = valid && !(mxq < a.thr);  // fock_build_non_diag.f90:69
-    const bool jonly = a.jonly != 0;
-    const int nsh = a.nsh;
-    const int sO = S == 0 ? bra.sa : bra.sb, sX = S == 0 ? bra.sb : bra.sa;
-    const int O0 = S == 0 ? bra.aoa : bra.aob, X0 = S == 0 ? bra.aob : bra.aoa;
-    const int c0 = ket.aoa, d0 = ket.aob;
-    // density blocks in shell-pair order, row-major within a block
-    const double* __restrict__ Pb = a.Pb;
-    const double* __restrict__ Bab = Pb + __ldg(a.boff + bra.sa * nsh + bra.sb);
-    const double* __restrict__ BOc = Pb + __ldg(a.boff + sO * nsh + ket.sa);
-    const double* __restrict__ BOd = Pb + __ldg(a.boff + sO * nsh + ket.sb);
-    const double* __restrict__ BXc = Pb + __ldg(a.boff + sX * nsh + ket.sa);
-    const double* __restrict__ BXd = Pb + __ldg(a.boff + sX * nsh + ket.sb);
-    const double* __restrict__ Bcd = Pb + __ldg(a.boff + ket.sa * nsh + ket.sb);
-    extern __shared__ __align__(16) double hf_scatg_smem[];
-    E* eb = reinterpret_cast<E*>(hf_scatg_smem) + tid;                 // [NBUF][SLAB][T], own column
-    E* sp = reinterpret_cast<E*>(hf_scatg_smem) + NBUF * SLAB * T + ql;  // [NPS][QB]: P_cd, P_Xc, P_Xd
-    const E* __restrict__ e = reinterpret_cast<const E*>(a.out) + tcol(tq, NA * NB * NC * ND);
-    const size_t st = TQ;
-    auto issue = [&](int x) {
-        if (x < NX) {
-            const E* src = e + (size_t)((S == 0 ? g * NB + x : x * NB + g) * SLAB) * st;
-            E* dst = eb + (x % NBUF) * SLAB * T;
-#pragma unroll
-            for (int r = 0; r < SLAB; ++r) cp_async_elem(dst + r * T, src + (size_t)r * st);
-        }
-        cp_async_commit();  // empty groups keep the count uniform
-    };
-    issue(0);
-    // the quartet's P_cd, P_Xc and P_Xd, loaded once by its four lanes
-    for (int v = g; v < NPS; v += SG)
-        sp[v * QB] = (E)__ldg(v < SLAB ? Bcd + v : v < SLAB + NX * NC ? BXc + (v - SLAB) : BXd + (v - SLAB - NX * NC));
-    E poc[NC], pod[ND], pox[NX];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) poc[k] = (E)__ldg(BOc + g * NC + k);
-#pragma unroll
-    for (int l = 0; l < ND; ++l) pod[l] = (E)__ldg(BOd + g * ND + l);
-#pragma unroll
-    for (int x = 0; x < NX; ++x) pox[x] = (E)__ldg(Bab + (S == 0 ? g * NB + x : x * NB + g));
-    __syncwarp();
-    // warp-uniform shells: a block element with one address for the whole
-    // warp is summed over the warp's eight quartets and added by one lane
-    auto same = [](int x) { return __all_sync(0xffffffffu, x == __shfl_sync(0xffffffffu, x, 0)); };
-    const bool ua = same(bra.aoa), ub = same(bra.aob), uc = same(c0), ud = same(d0);
-    const bool uO = S == 0 ? ua : ub, uX = S == 0 ? ub : ua;
-    auto Ga = [&](int r, int c) { return a.G + r + (size_t)c * a.nb; };
-    // `shuf` is warp-uniform (every lane runs the shuffles); `uni` may differ
-    // between lanes of different g but is the same for lanes of equal g,
-    // which are the lanes the shuffles sum over
-    auto emit = [&](double* addr, double v, bool shuf, bool uni, bool has) {
-        double r = v;
-        if (shuf) {
-            r += __shfl_xor_sync(0xffffffffu, r, 4);
-            r += __shfl_xor_sync(0xffffffffu, r, 8);
-            r += __shfl_xor_sync(0xffffffffu, r, 16);
-        }
-        if (uni) {
-            if (lane < SG && has) atomicAdd(addr, r);
-        } else if (act && has) {
-            atomicAdd(addr, v);
-        }
-    };
-    const double s = (bra.sa == bra.sb ? 0.5 : 1.0) * (ket.sa == ket.sb ? 0.5 : 1.0);
-    const double s2 = 2.0 * s, hs = -0.5 * s;
-    E koc[NC], kod[ND], jcd[NJ4];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) koc[k] = 0;
-#pragma unroll
-    for (int l = 0; l < ND; ++l) kod[l] = 0;
-#pragma unroll
-    for (int v = 0; v < NJ4; ++v) jcd[v] = 0;
-#pragma unroll
-    for (int x = 0; x < NX; ++x) {
-        issue(x + 1);
-        cp_async_wait<NBUF - 1>();  // this thread's copies of slab x have landed
-        const E* es = eb + (x % NBUF) * SLAB * T;
-        E pxd[ND], kx[NK4], jox = 0;
-#pragma unroll
-        for (int l = 0; l < ND; ++l) pxd[l] = sp[(SLAB + NX * NC + x * ND + l) * QB];
-#pragma unroll
-        for (int v = 0; v < NK4; ++v) kx[v] = 0;
-#pragma unroll
-        for (int k = 0; k < NC; ++k) {
-            const E pxc = sp[(SLAB + x * NC + k) * QB];
-#pragma unroll
-            for (int l = 0; l < ND; ++l) {
-                const E v = es[(k * ND + l) * T];
-                jox += sp[(k * ND + l) * QB] * v;
-                jcd[k * ND + l] += pox[x] * v;
-                if (!jonly) {
-                    koc[k] += pxd[l] * v;
-                    kod[l] += pxc * v;
-                    kx[k] += pod[l] * v;       // K_Xc[x][k]
-                    kx[NC + l] += poc[k] * v;  // K_Xd[x][l]
-                }
-            }
-        }
-        emit(S == 0 ? Ga(O0 + g, X0 + x) : Ga(X0 + x, O0 + g), act ? s2 * (double)jox : 0.0, ua && ub, ua && ub,
-             true);
-        if (!jonly) {
-            const int base = group_reduce_scatter<NK4>(kx, g);
-            const bool shuf = uX && (uc || ud);  // warp-uniform
-#pragma unroll
-            for (int v = 0; v < NK4 / 4; ++v) {
-                const int y = base + v;
-                const bool isc = y < NC;
-                emit(Ga(X0 + x, isc ? c0 + y : d0 + (y - NC)), act && y < NK ? hs * (double)kx[v] : 0.0, shuf,
-                     uX && (isc ? uc : ud), y < NK);
-            }
-        }
-    }
-    cp_async_wait<0>();
-    if (!jonly) {
-#pragma unroll
-        for (int k = 0; k < NC; ++k)
-            emit(Ga(O0 + g, c0 + k), act ? hs * (double)koc[k] : 0.0, uO && uc, uO && uc, true);
-#pragma unroll
-        for (int l = 0; l < ND; ++l)
-            emit(Ga(O0 + g, d0 + l), act ? hs * (double)kod[l] : 0.0, uO && ud, uO && ud, true);
-    }
-    {
-        const int base = group_reduce_scatter<NJ4>(jcd, g);
-#pragma unroll
-        for (int v = 0; v < NJ4 / 4; ++v) {
-            const int y = base + v;
-            emit(Ga(c0 + y / ND, d0 + y % ND), act && y < NC * ND ? s2 * (double)jcd[v] : 0.0, uc && ud, uc && ud,
-                 y < NC * ND);
-        }
-    }
-    if (a.stats) {  // counted once per quartet, by its lane 0
-        const unsigned long long nsc = act && g == 0 ? 1ull : 0ull;
-        const unsigned long long npr = valid && g == 0 ? (unsigned long long)(bra.np * ket.np) : 0ull;
-        warp_add_stats(a.stats, nsc, npr, a.f32 ? nsc : 0ull);
-    }
 }
 
 // Small chunks: one warp per quartet, its block in shared memory and the
@@ -857,7 +681,7 @@ __global__ void __launch_bounds__(ND_THREADS, scatg_minb(S == 0 ? NB : NA, NC, N
 // serial chain of 100-625 row loads; at a few hundred quartets that chain is
 // the kernel's time (25-100 us), while this form takes a few us.  It reads
 // each element six times from shared memory, so chunks that fill the SMs keep
-// the one-thread and grouped forms.
+// the one-thread form.
 constexpr int WPB = ND_THREADS / 32;  // quartets per block
 template <int NA, int NB, int NC, int ND, typename E>
 __global__ void __launch_bounds__(ND_THREADS) k_scatter_warp(StagedArgs a) {
@@ -881,7 +705,8 @@ __global__ void __launch_bounds__(ND_THREADS) k_scatter_warp(StagedArgs a) {
         if (!__any_sync(0xffffffffu, !(m < a.thr))) continue;  // fock_build_non_diag.f90:69
         ++nsc;
         const double s = (bra.sa == bra.sb ? 0.5 : 1.0) * (ket.sa == ket.sb ? 0.5 : 1.0);
-        scatter_lanes<NA, NB, NC, ND>(se[wp], sw[wp], s, bra, ket, a.P, a.G, a.nb, a.jonly != 0, lane, 32);
+        scatter_lanes<NA, NB, NC, ND>(se[wp], sw[wp], s, bra, ket, a.P, a.nb, BlockDst{a.G, a.boff, a.nsh},
+                                      a.jonly != 0, lane, 32);
     }
     if (a.stats && lane == 0 && npr) {
         atomicAdd(&a.stats->prim, npr);
@@ -917,7 +742,8 @@ __global__ void __launch_bounds__(ND_THREADS) k_scatter_diag(StagedArgs a) {
         se[wp][i] = fabs(v) > INTTHRESH ? v : 0.0;  // element skip
     }
     const double f = pr.sa == pr.sb ? 1.0 : 2.0;
-    scatter_lanes<NA, NB, NA, NB>(se[wp], sw[wp], f * f / 8.0, pr, pr, a.P, a.G, a.nb, false, lane, 32);
+    scatter_lanes<NA, NB, NA, NB>(se[wp], sw[wp], f * f / 8.0, pr, pr, a.P, a.nb, BlockDst{a.G, a.boff, a.nsh}, false,
+                                  lane, 32);
 }
 
 typedef void (*NDKernel)(NDArgs);
@@ -942,11 +768,6 @@ struct ClassKernels {
     StagedKernel scat32;          // scatter of FP32 chunks (float rows), or nullptr
     int scat32_smem;
     StagedKernel scatw, scatw32;  // small chunks: one warp per quartet
-    // grouped scatter (four lanes per quartet) where a bra shell has four
-    // functions, else nullptr
-    StagedKernel scatg, scatg32;
-    int scatg_smem, scatg32_smem;
-    int grp64, grp32;             // the grouped scatter is the default for FP64 / FP32 chunks
     // every role of a stage in one launch (gridDim.y = roles), for small
     // chunks; the primitive-loop stages (ma, and mb of mode 1) run on work units
     StagedKernel ma64, ma32;      // stage-A roles (staged3)

@@ -675,25 +675,6 @@ __global__ void __launch_bounds__(RB_THREADS, {minb} * RB_SCALE) {kname}(StagedA
 }}"""
 
 
-def grouped_scatter_reg(NA: int, NB: int, NC: int, ND: int, prm: dict) -> str:
-    """Registration of the grouped scatter (four lanes per quartet, lane g
-    owning function g of a four-function bra shell: the first shell when it
-    has four functions, else the second), or nullptr when neither has.
-    scat_grouped64 / scat_grouped32 in the tuning table choose it by default
-    for the FP64 / FP32 chunks of the class (measured per class)."""
-    S = 0 if NA == 4 else 1 if NB == 4 else -1
-    if S < 0:
-        return ("    k->scatg = nullptr;\n    k->scatg32 = nullptr;\n"
-                "    k->scatg_smem = 0;\n    k->scatg32_smem = 0;\n    k->grp64 = 0;\n    k->grp32 = 0;")
-    NX = NB if S == 0 else NA
-    return (f"    k->scatg = k_scatter_grouped<{NA}, {NB}, {NC}, {ND}, {S}>;\n"
-            f"    k->scatg_smem = scatg_smem_bytes({NX}, {NC}, {ND}, 8);\n"
-            f"    k->scatg32 = k_scatter_grouped<{NA}, {NB}, {NC}, {ND}, {S}, float>;\n"
-            f"    k->scatg32_smem = scatg_smem_bytes({NX}, {NC}, {ND}, 4);\n"
-            f"    k->grp64 = {int(bool(prm.get('scat_grouped64', False)))};\n"
-            f"    k->grp32 = {int(bool(prm.get('scat_grouped32', False)))};")
-
-
 def class_source(ci: int, bi: int, ki: int):
     """Header (device functions) and translation unit (kernels) of one
     quartet class; returns (cuh_text, cu_text, info).
@@ -801,7 +782,6 @@ __global__ void __launch_bounds__(RB_THREADS, {prm["minb32"] if f32 else 2} * RB
                    f"    k->scat32_smem = scat_smem_bytes({NA}, {NB}, {NC}, {ND}, 4);\n"
                    f"    k->scatw = k_scatter_warp<{NA}, {NB}, {NC}, {ND}, double>;\n"
                    f"    k->scatw32 = k_scatter_warp<{NA}, {NB}, {NC}, {ND}, float>;")
-        reg.append(grouped_scatter_reg(NA, NB, NC, ND, prm))
         if bi == ki:
             reg.append(f"    k->diag0 = nullptr;\n    k->diag1 = nullptr;")
             reg.append(f"    k->dscat0 = k_scatter_diag<{NA}, {NB}, 0>;\n    k->dscat1 = k_scatter_diag<{NA}, {NB}, 1>;")
@@ -888,7 +868,6 @@ __global__ void __launch_bounds__(RB_THREADS, RB_SCALE) {kname}(StagedArgs a) {{
                    f"    k->scat32_smem = scat_smem_bytes({NA}, {NB}, {NC}, {ND}, 4);\n"
                    f"    k->scatw = k_scatter_warp<{NA}, {NB}, {NC}, {ND}, double>;\n"
                    f"    k->scatw32 = k_scatter_warp<{NA}, {NB}, {NC}, {ND}, float>;")
-        reg.append(grouped_scatter_reg(NA, NB, NC, ND, prm))
         if bi == ki:
             reg.append(f"    k->diag0 = nullptr;\n    k->diag1 = nullptr;")
             reg.append(f"    k->dscat0 = k_scatter_diag<{NA}, {NB}, 0>;\n    k->dscat1 = k_scatter_diag<{NA}, {NB}, 1>;")
@@ -1001,7 +980,8 @@ def main(outdir: str):
         lines.append(f"inline int host_scatter_{ci}(const double* e, double s, const GPair& b, const GPair& k,")
         lines.append(f"                             const double* P, double* G, int nb, bool jonly) {{")
         lines.append(f"    double w[scatter_dens({na}, {nb_}, {nc}, {nd})];")
-        lines.append(f"    scatter_lanes<{na}, {nb_}, {nc}, {nd}>(e, w, s, b, k, P, G, nb, jonly, 0, 1);")
+        lines.append("    auto at = [&](int, int, int r, int c, int) { return G + r + (size_t)c * nb; };")
+        lines.append(f"    scatter_lanes<{na}, {nb_}, {nc}, {nd}>(e, w, s, b, k, P, nb, at, jonly, 0, 1);")
         lines.append("    return 0;")
         lines.append("}")
     lines.append("typedef void (*HostEri)(const GPair&, const GPair&, const PrimSoA&, const double*, const float*, double*, int);")

@@ -342,11 +342,13 @@ __global__ void k_fma_peak(T* out, int iters, T a, T b) {
     if (s == (T)-1.2345) out[0] = s;  // keeps the chains live
 }
 
-__global__ void k_symm(double* __restrict__ F, const double* __restrict__ G, int nb) {
+// F += G + G^T; G is in the shell-pair blocks of k_pblock.
+__global__ void k_symm(double* __restrict__ F, const double* __restrict__ G, const int2* __restrict__ aomap,
+                       const int* __restrict__ nfsh, const int* __restrict__ boff, int nb, int nsh) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)nb * nb) return;
-    const int i = (int)(t % nb), j = (int)(t / nb);
-    F[t] += G[t] + G[j + (size_t)i * nb];
+    const int2 r = aomap[t % nb], c = aomap[t / nb];
+    F[t] += G[boff[r.x * nsh + c.x] + r.y * nfsh[c.x] + c.y] + G[boff[c.x * nsh + r.x] + c.y * nfsh[r.x] + r.y];
 }
 
 // ------------------------------------------------------------- host ----
@@ -368,7 +370,6 @@ struct hfgpu_handle {
     int timing = 0;
     int device = 0;                       // the CUDA device current at hfgpu_init
     long long merge_blocks = 0;           // chunks up to this many role blocks run one launch per stage
-    int grouped_scatter = 1;              // four-lane scatter: 1 per class tuning, 2 everywhere, 0 nowhere
     int nstreams = 4;                     // class streams the off-diagonal build uses (<= NSTREAM)
     cudaStream_t stream = nullptr;
     cudaStream_t aux[NSTREAM] = {};    // independent classes run concurrently on these
@@ -494,10 +495,6 @@ struct ClassTable {
                 cudaFuncSetAttribute(k[c].scat, cudaFuncAttributeMaxDynamicSharedMemorySize, k[c].scat_smem);
             if (k[c].scat32 && k[c].scat32_smem > 0)
                 cudaFuncSetAttribute(k[c].scat32, cudaFuncAttributeMaxDynamicSharedMemorySize, k[c].scat32_smem);
-            if (k[c].scatg && k[c].scatg_smem > 0)
-                cudaFuncSetAttribute(k[c].scatg, cudaFuncAttributeMaxDynamicSharedMemorySize, k[c].scatg_smem);
-            if (k[c].scatg32 && k[c].scatg32_smem > 0)
-                cudaFuncSetAttribute(k[c].scatg32, cudaFuncAttributeMaxDynamicSharedMemorySize, k[c].scatg32_smem);
             // The role kernels use no shared memory: they prefer the largest
             // L1 carve-out (HFGPU_CARVEOUT=<percent of shared memory> or
             // "none" overrides).  With the four class streams, where role and
@@ -563,7 +560,8 @@ int launch_maxdm(hfgpu_handle* h, const double* P, double* md = nullptr) {
 int launch_symm(hfgpu_handle* h, double* F, const double* G = nullptr) {
     long long n = (long long)h->nb * h->nb;
     ++h->launches;
-    k_symm<<<(int)((n + 255) / 256), 256, 0, h->stream>>>(F, G ? G : h->d_G, h->nb);
+    k_symm<<<(int)((n + 255) / 256), 256, 0, h->stream>>>(F, G ? G : h->d_G, h->d_aomap, h->d_nfsh, h->d_boff, h->nb,
+                                                          h->nsh);
     HF_CHECK(cudaGetLastError());
     return HFGPU_OK;
 }
@@ -604,6 +602,7 @@ int run_staged_diag(hfgpu_handle* h, int t, int mode, const double* P, double th
         a.nroles = K.nrole_b;
         a.P = P;
         a.G = G;
+        a.boff = h->d_boff;
         a.nb = h->nb;
         a.thr = thr;
         a.stats = nullptr;
@@ -640,7 +639,7 @@ int launch_diag(hfgpu_handle* h, int mode, const double* P, double thr, double* 
             if (rc) return rc;
             continue;
         }
-        DiagArgs a{h->d_pairs[t], n, h->psoa, h->d_boys, h->d_schw[t], md, h->nsh, P, G, h->nb, thr};
+        DiagArgs a{h->d_pairs[t], n, h->psoa, h->d_boys, h->d_schw[t], md, h->nsh, P, G, h->d_boff, h->nb, thr};
         ++h->launches;
         diag_kernel(t, mode)<<<(n + WPB - 1) / WPB, ND_THREADS, 0, s_direct>>>(a);
         HF_CHECK(cudaGetLastError());
@@ -981,16 +980,9 @@ int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, d
             }
         }
         ++h->launches;
-        // grouped scatter: where the class's tuning chooses it (grouped_scatter 1),
-        // everywhere it exists (2) or nowhere (0)
-        const bool grp = h->grouped_scatter == 2 || (h->grouped_scatter == 1 && (prec ? K.grp32 : K.grp64));
-        const StagedKernel sg = grp ? (prec ? K.scatg32 : K.scatg) : nullptr;
         if (m <= h->warp_scatter) {  // one warp per quartet
             const unsigned wblocks = walk_blocks((m + WPB - 1) / WPB, 8LL * h->nsm, capture);
             (prec ? K.scatw32 : K.scatw)<<<wblocks, ND_THREADS, 0, stream>>>(a);
-        } else if (sg) {  // four lanes per quartet
-            const int gblocks = (int)(((long long)m * SG + ND_THREADS - 1) / ND_THREADS);
-            sg<<<gblocks, ND_THREADS, prec ? K.scatg32_smem : K.scatg_smem, stream>>>(a);
         } else if (prec && K.scat32) {
             K.scat32<<<blocks, ND_THREADS, K.scat32_smem, stream>>>(a);  // float rows
         } else {
@@ -1102,9 +1094,10 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
             a.prims = h->apsoa;
             a.boys = h->d_boys;
             a.boysf = h->d_boysf;
-            a.P = P;
+            a.Pb = h->d_Pb;
             a.G = h->d_G;
-            a.nb = h->nb;
+            a.boff = h->d_boff;
+            a.nsh = h->nsh;
             a.thr = thr;
             a.jonly = jonly;
             a.stats = h->d_stats + c;
@@ -1188,8 +1181,6 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
         h->warp_scatter = 16LL * h->nsm;
         if (const char* e = getenv("HFGPU_WARP_SCATTER")) h->warp_scatter = atoll(e);
         if (const char* e = getenv("HFGPU_STREAMS")) h->nstreams = std::max(1, std::min(NSTREAM, atoi(e)));
-        if (const char* e = getenv("HFGPU_SCATTER"))  // "single" / "grouped" override the per-class choice
-            h->grouped_scatter = strcmp(e, "single") == 0 ? 0 : strcmp(e, "grouped") == 0 ? 2 : 1;
     }
     int rc = 0;
     const size_t nb2 = (size_t)h->nb * h->nb;
