@@ -190,8 +190,8 @@ struct ClassStats {
 // pairs from one group of the ket list, so that every quartet in the
 // compacted sub-list runs its primitive loops with the same trip counts.
 struct ScreenSub {
-    long long start;   // first padded candidate index
-    long long ncand;   // candidates (unpadded)
+    long long ncand;   // candidates
+    int tile0;         // first screening tile
     int cls;
     int same;          // one group against itself: pairs i > j only
     int b0, nbra;      // bra range in the active list

@@ -146,10 +146,18 @@ __global__ void k_maxdm(const int* __restrict__ shtyp, const int* __restrict__ a
     md[(size_t)b * nsh + a] = m;
 }
 
+// Screening tiles: `tw` words of 32 consecutive candidates of one sub-class,
+// one warp's work, a word at a time.  Large systems take 64 words (a lane
+// keeps two mask words); small ones fewer, so that there are warps enough:
+// with 64 words (H2O)12 has 2200 tiles, 15 warps per SM, each a serial chain
+// (60 us, the whole screen's time).
+constexpr int TWORDS_MAX = 64, TWORDS_MIN = 8;
+
 struct ScreenArgs {
     const ScreenSub* subs;
     int nsub;
-    long long ntot;
+    int ntile;
+    int tw;                   // words per tile
     const int2* sh[NPT];      // (sa, sb) per active pair, per pair type
     const double* schw[NPT];  // Schwarz factor per active pair
     const double* md;
@@ -157,72 +165,154 @@ struct ScreenArgs {
     double thr;
     int jonly;
     double f32cut;
-    unsigned long long* cnt;  // [2*nsub]: pass 1 counts, pass 2 positions
+    unsigned long long* cnt;  // [2*nsub] survivors per sub-class (FP64, FP32)
+    int* tcnt;                // [2*ntile] survivors per tile; after k_offsets the entries before it in its sub-class
+    unsigned* mask;           // [tw] survivors per tile, then (f32cut > 0) the FP32 ones of every tile
     uint2* qbuf;
 };
 
+// The sub-class of a tile: the last one whose first tile is <= t.
+__device__ __forceinline__ int tile_sub(const ScreenArgs& a, int t) {
+    int lo = 0, hi = a.nsub - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (a.subs[mid].tile0 <= t) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// Candidate u of a sub-class as (bra, ket) within its two groups, row by row.
+__device__ __forceinline__ void candidate(const ScreenSub& S, long long u, int& i, int& j) {
+    long long r;
+    if (S.same) {
+        r = (long long)((1.0 + sqrt(1.0 + 8.0 * (double)u)) * 0.5);
+        while (r * (r - 1) / 2 > u) --r;
+        while ((r + 1) * r / 2 <= u) ++r;
+        j = (int)(u - r * (r - 1) / 2);
+    } else {
+        r = u / S.nket;
+        j = (int)(u - r * S.nket);
+    }
+    i = (int)r;
+}
+
+// 32 candidates further.
+__device__ __forceinline__ void advance(const ScreenSub& S, int& i, int& j) {
+    j += 32;
+    if (S.same) {
+        while (j >= i) j -= i++;
+    } else if (S.nket >= 32) {
+        if (j >= S.nket) {
+            j -= S.nket;
+            ++i;
+        }
+    } else {
+        i += j / S.nket;
+        j %= S.nket;
+    }
+}
+
 // Per-quartet screen of fock_build_non_diag.f90:63-67 over every candidate
-// pair of active shell pairs.  PASS 0 counts the survivors of each
-// sub-class (FP64 and FP32 separately); PASS 1 writes them compacted at the
-// offsets the host derived from those counts.  Candidates of each sub-class
-// are padded to a multiple of 32 so a warp never spans two sub-classes.
-template <int PASS>
-__global__ void k_screen(ScreenArgs a) {
+// pair of active shell pairs, one warp per tile: the survivors as a bit mask
+// and their counts.  Bound by the five density gathers of a candidate (L1);
+// one search and one division per tile instead of one per 32 candidates, and
+// a second pass that expands the masks instead of screening again, took the
+// two passes from 1.71 + 1.98 ms to 0.95 + 0.45 ms on C60 (4.2e8 candidates).
+__global__ void __launch_bounds__(256) k_screen(ScreenArgs a) {
     const int lane = threadIdx.x & 31;
-    const long long nwarps_total = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long w = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); w * 32 < a.ntot;
-         w += nwarps_total) {
-        const long long w0 = w * 32;
-        int lo_i = 0, hi_i = a.nsub - 1;  // last sub with start <= w0
-        while (lo_i < hi_i) {
-            const int mid = (lo_i + hi_i + 1) >> 1;
-            if (a.subs[mid].start <= w0) lo_i = mid;
-            else hi_i = mid - 1;
-        }
-        const int c = lo_i;
-        const ScreenSub S = a.subs[c];
-        const long long u = w0 + lane - S.start;
-        bool pass = false, lo = false;
-        unsigned ii = 0, jj = 0;
-        if (u < S.ncand) {
-            long long i, j;
-            if (S.same) {
-                i = (long long)((1.0 + sqrt(1.0 + 8.0 * (double)u)) * 0.5);
-                while (i * (i - 1) / 2 > u) --i;
-                while ((i + 1) * i / 2 <= u) ++i;
-                j = u - i * (i - 1) / 2;
-            } else {
-                i = u / S.nket;
-                j = u - i * S.nket;
-            }
-            ii = (unsigned)(S.b0 + i);
-            jj = (unsigned)(S.k0 + j);
-            const int2 ab = a.sh[CLS_BI[S.cls]][ii], cd = a.sh[CLS_KI[S.cls]][jj];
-            const double dc = fmax(a.md[ab.x * a.nsh + ab.y], a.md[cd.x * a.nsh + cd.y]);
-            double v = dc;
+    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (t >= a.ntile) return;
+    const int c = tile_sub(a, t);
+    const ScreenSub S = a.subs[c];
+    const int bi = CLS_BI[S.cls], ki = CLS_KI[S.cls];
+    const long long u0 = (long long)(t - S.tile0) * (32 * a.tw);
+    const int left = (int)min((long long)(32 * a.tw), S.ncand - u0), words = (left + 31) >> 5;
+    const int2* __restrict__ bsh = a.sh[bi] + S.b0;
+    const int2* __restrict__ ksh = a.sh[ki] + S.k0;
+    const double* __restrict__ bsw = a.schw[bi] + S.b0;
+    const double* __restrict__ ksw = a.schw[ki] + S.k0;
+    const double* __restrict__ md = a.md;
+    const int nsh = a.nsh;
+    int i, j;
+    candidate(S, u0 + lane, i, j);
+    unsigned m[2] = {0, 0}, lo[2] = {0, 0};  // words lane and lane + 32
+    for (int w = 0; w < words; ++w) {
+        bool pass = false, low = false;
+        if (w * 32 + lane < left) {
+            const int2 ab = __ldg(bsh + i), cd = __ldg(ksh + j);
+            double v = fmax(__ldg(md + ab.x * nsh + ab.y), __ldg(md + cd.x * nsh + cd.y));
             if (!a.jonly) {
-                const double dx = fmax(fmax(a.md[ab.x * a.nsh + cd.x], a.md[ab.x * a.nsh + cd.y]),
-                                       fmax(a.md[ab.y * a.nsh + cd.x], a.md[ab.y * a.nsh + cd.y]));
-                v = fmax(dc, 0.25 * dx);
+                const double* __restrict__ ra = md + ab.x * nsh;
+                const double* __restrict__ rb = md + ab.y * nsh;
+                const double dx = fmax(fmax(__ldg(ra + cd.x), __ldg(ra + cd.y)),
+                                       fmax(__ldg(rb + cd.x), __ldg(rb + cd.y)));
+                v = fmax(v, 0.25 * dx);
             }
-            const double bound = a.schw[CLS_BI[S.cls]][ii] * a.schw[CLS_KI[S.cls]][jj] * v;
+            const double bound = __ldg(bsw + i) * __ldg(ksw + j) * v;
             pass = !(bound < a.thr);
-            lo = pass && bound < a.f32cut;
+            low = pass && bound < a.f32cut;
         }
-        const unsigned m64 = __ballot_sync(0xffffffffu, pass && !lo);
-        const unsigned m32 = __ballot_sync(0xffffffffu, lo);
-        unsigned long long b64 = 0, b32 = 0;
-        if (lane == 0) {
-            if (m64) b64 = atomicAdd(&a.cnt[2 * c], (unsigned long long)__popc(m64));
-            if (m32) b32 = atomicAdd(&a.cnt[2 * c + 1], (unsigned long long)__popc(m32));
+        const unsigned mw = __ballot_sync(0xffffffffu, pass), lw = __ballot_sync(0xffffffffu, low);
+        if (lane == (w & 31)) {
+            if (w < 32) m[0] = mw, lo[0] = lw;
+            else m[1] = mw, lo[1] = lw;
         }
-        if (PASS == 1) {
-            b64 = __shfl_sync(0xffffffffu, b64, 0);
-            b32 = __shfl_sync(0xffffffffu, b32, 0);
-            const unsigned lt = (1u << lane) - 1u;
-            if (pass && !lo) a.qbuf[S.off[0] + (long long)b64 + __popc(m64 & lt)] = make_uint2(ii, jj);
-            if (lo) a.qbuf[S.off[1] + (long long)b32 + __popc(m32 & lt)] = make_uint2(ii, jj);
+        advance(S, i, j);
+    }
+    const size_t at = (size_t)t * a.tw + lane;
+    unsigned* ml = a.mask + (size_t)a.ntile * a.tw;
+    for (int x = 0; x < 2; ++x)
+        if (lane + 32 * x < a.tw) {
+            a.mask[at + 32 * x] = m[x];
+            if (a.f32cut > 0.0) ml[at + 32 * x] = lo[x];
         }
+    int n32 = __popc(lo[0]) + __popc(lo[1]), n64 = __popc(m[0]) + __popc(m[1]) - n32;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        n64 += __shfl_xor_sync(0xffffffffu, n64, o);
+        n32 += __shfl_xor_sync(0xffffffffu, n32, o);
+    }
+    if (lane < 2) a.tcnt[2 * t + lane] = lane ? n32 : n64;
+    if (lane == 0 && n64) atomicAdd(&a.cnt[2 * c], (unsigned long long)n64);
+    if (lane == 1 && n32) atomicAdd(&a.cnt[2 * c + 1], (unsigned long long)n32);
+}
+
+// The compacted lists from the masks, one warp per tile.  The entries of a
+// sub-class are in candidate order: a warp's 32 quartets share their bra pair
+// and mostly the ket's first shell.
+__global__ void __launch_bounds__(256) k_expand(ScreenArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (t >= a.ntile) return;
+    const size_t at = (size_t)t * a.tw + lane;
+    const unsigned* ml = a.mask + (size_t)a.ntile * a.tw;
+    unsigned m[2] = {0, 0}, lo[2] = {0, 0};
+    for (int x = 0; x < 2; ++x)
+        if (lane + 32 * x < a.tw) {
+            m[x] = a.mask[at + 32 * x];
+            if (a.f32cut > 0.0) lo[x] = ml[at + 32 * x];
+        }
+    if (!__any_sync(0xffffffffu, m[0] | m[1])) return;
+    const int c = tile_sub(a, t);
+    const ScreenSub S = a.subs[c];
+    const long long u0 = (long long)(t - S.tile0) * (32 * a.tw);
+    long long o64 = S.off[0] + a.tcnt[2 * t], o32 = S.off[1] + a.tcnt[2 * t + 1];
+    int i, j;
+    candidate(S, u0 + lane, i, j);
+    const int words = (int)((min((long long)(32 * a.tw), S.ncand - u0) + 31) >> 5);
+    const unsigned lt = (1u << lane) - 1u;
+    for (int w = 0; w < words; ++w) {
+        const unsigned mw = __shfl_sync(0xffffffffu, w < 32 ? m[0] : m[1], w & 31);
+        const unsigned lw = __shfl_sync(0xffffffffu, w < 32 ? lo[0] : lo[1], w & 31), hw = mw & ~lw;
+        if (mw >> lane & 1) {
+            const uint2 q = make_uint2((unsigned)(S.b0 + i), (unsigned)(S.k0 + j));
+            if (lw >> lane & 1) a.qbuf[o32 + __popc(lw & lt)] = q;
+            else a.qbuf[o64 + __popc(hw & lt)] = q;
+        }
+        o64 += __popc(hw);
+        o32 += __popc(lw);
+        advance(S, i, j);
     }
 }
 
@@ -233,6 +323,7 @@ struct OffsetArgs {
     long long coff[NCLS];    // first entry of class c in the quartet buffer
     float fill[NCLS][2];     // threads that fill the GPU with this class's kernel, per role (FP64, FP32)
     int lmin[NCLS];          // fewest primitive quartets a lane is given
+    int tw;                  // words per screening tile
 };
 
 // Fewest lanes (lgb + lgk) over npb x npk primitives with at most `most`
@@ -261,17 +352,54 @@ __device__ __forceinline__ long long warp_scan(long long v, int lane) {  // incl
     return v;
 }
 
-// Write offsets of the compacted lists from the pass-0 counts, on the device
+// Exclusive sums of a sub-class's tile counts (FP64 and FP32), by one block.
+constexpr int OFF_THREADS = 128;
+__device__ __forceinline__ void scan_tiles(const ScreenSub& S, int tw, int* __restrict__ tcnt) {
+    __shared__ int part[OFF_THREADS / 32][2];
+    const int nt = (int)((S.ncand + 32 * tw - 1) / (32 * tw)), lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    int2* __restrict__ t = reinterpret_cast<int2*>(tcnt) + S.tile0;
+    int2 run = make_int2(0, 0);
+    for (int k0 = 0; k0 < nt; k0 += OFF_THREADS) {
+        const int k = k0 + (int)threadIdx.x;
+        const int2 v = k < nt ? t[k] : make_int2(0, 0);
+        int2 s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, s.x, o), y = __shfl_up_sync(0xffffffffu, s.y, o);
+            if (lane >= o) s.x += x, s.y += y;
+        }
+        if (lane == 31) part[wp][0] = s.x, part[wp][1] = s.y;
+        __syncthreads();
+        int2 before = run;
+        for (int q = 0; q < OFF_THREADS / 32; ++q) {
+            if (q < wp) before.x += part[q][0], before.y += part[q][1];
+            run.x += part[q][0], run.y += part[q][1];
+        }
+        if (k < nt) t[k] = make_int2(before.x + s.x - v.x, before.y + s.y - v.y);
+        __syncthreads();
+    }
+}
+
+// Write offsets of the compacted lists from the screen's counts, on the device
 // so that a build needs no host round trip: per class its FP64 entries, then
 // its FP32 entries, sub-classes in order.  Also stores the per-class totals
 // that the class kernels read, and cuts each list into work units (see Unit):
 // a quartet is spread over as many lanes as it takes for a lane's share of
 // its primitive loops to be near the class's primitive work over the threads
 // that fill the GPU, and at least lmin.  A class that fills the GPU anyway
-// keeps one lane per quartet.  One warp per class.
-__global__ void k_offsets(OffsetArgs o, ScreenSub* __restrict__ subs, const unsigned long long* __restrict__ cnt,
-                          unsigned long long* __restrict__ ncls, int* __restrict__ nunit) {
+// keeps one lane per quartet.  The first NCLS blocks take one class each (one
+// warp); the others turn the tile counts of one sub-class each into the
+// entries before the tile.
+__global__ void __launch_bounds__(OFF_THREADS) k_offsets(OffsetArgs o, ScreenSub* __restrict__ subs,
+                                                         const unsigned long long* __restrict__ cnt,
+                                                         int* __restrict__ tcnt, unsigned long long* __restrict__ ncls,
+                                                         int* __restrict__ nunit) {
     const int c = blockIdx.x, lane = threadIdx.x;
+    if (c >= NCLS) {
+        scan_tiles(subs[c - NCLS], o.tw, tcnt);
+        return;
+    }
+    if (lane >= 32) return;
     const int k0 = o.csub[c], k1 = o.csub[c + 1];
     long long n[2] = {0, 0};
     double work[2] = {0.0, 0.0};
@@ -411,10 +539,13 @@ struct hfgpu_handle {
     size_t scratch_budget = 0;     // bytes; 0 = default (HFGPU_SCRATCH_MB, or 24 GiB capped at device memory / 6)
     size_t naprims = 0;            // primitive pairs of the active lists
     unsigned long long* d_cnt = nullptr;
+    unsigned* d_mask = nullptr;    // survivor masks of the screening tiles (all, then the FP32 ones)
+    int* d_tcnt = nullptr;         // survivors per tile (FP64, FP32)
+    size_t tilecap = 0, maskcap = 0;  // tiles and mask words the two hold
     ClassStats* d_stats = nullptr;
     // last build statistics
     double st_ms[NCLS] = {};
-    long long ntot = 0;
+    int ntile = 0;                  // screening tiles
     long long ccap[NCLS] = {};      // candidates per class (upper bound of its list)
     long long coff[NCLS] = {};      // class region in the quartet buffer
     long long n64[NCLS] = {}, n32[NCLS] = {};
@@ -797,7 +928,7 @@ int build_active(hfgpu_handle* h) {
         }
     }
     h->hsubs.clear();
-    long long start = 0, qoff = 0;
+    long long total_words = 0, qoff = 0;
     for (int c = 0; c < NCLS; ++c) {
         const int bi = CLASS_KERNELS[c].bi, ki = CLASS_KERNELS[c].ki;
         long long ccap = 0;
@@ -815,8 +946,7 @@ int build_active(hfgpu_handle* h) {
                 sub.npk = h->act_np[ki][sub.k0];
                 sub.ncand = sub.same ? (long long)sub.nbra * (sub.nbra - 1) / 2 : (long long)sub.nbra * sub.nket;
                 if (sub.ncand == 0) continue;
-                sub.start = start;
-                start += (sub.ncand + 31) / 32 * 32;
+                total_words += (sub.ncand + 31) / 32;
                 ccap += sub.ncand;
                 h->hsubs.push_back(sub);
             }
@@ -836,8 +966,28 @@ int build_active(hfgpu_handle* h) {
         h->offs.lmin[c] = K.mode == 0 ? LMIN_DIRECT : LMIN_STAGED;
     }
     h->offs.csub[0] = 0;
-    h->ntot = start;
+    // words per tile: the most that leaves 64 tiles per SM
+    int tw = TWORDS_MAX;
+    while (tw > TWORDS_MIN && total_words < 64LL * h->nsm * tw) tw /= 2;
+    long long tiles = 0;
+    for (ScreenSub& sub : h->hsubs) {
+        sub.tile0 = (int)tiles;
+        tiles += (sub.ncand + 32 * tw - 1) / (32 * tw);
+    }
+    h->offs.tw = tw;
+    if (tiles > (1LL << 30)) return set_err(HFGPU_ERR_UNSUPPORTED, "too many candidate quartets");
+    h->ntile = (int)tiles;
     total_q = qoff;
+    if ((size_t)tiles > h->tilecap || (size_t)tiles * tw > h->maskcap) {
+        dfree(h->d_mask, h->stream);
+        dfree(h->d_tcnt, h->stream);
+        h->tilecap = h->maskcap = 0;
+        int rc = dalloc(&h->d_mask, 2 * (size_t)tiles * tw, h->stream);
+        if (rc == HFGPU_OK) rc = dalloc(&h->d_tcnt, 2 * (size_t)tiles, h->stream);
+        if (rc) return rc;
+        h->tilecap = (size_t)tiles;
+        h->maskcap = (size_t)tiles * tw;
+    }
     if (h->hsubs.size() > h->subcap) {
         dfree(h->d_subs, h->stream);
         h->subcap = 0;
@@ -1005,11 +1155,12 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
     HF_CHECK(cudaMemsetAsync(h->d_ncls, 0, 3 * NCLS * sizeof(unsigned long long), h->stream));
     const int nsub = (int)h->hsubs.size();
     for (int c = 0; c < NCLS; ++c) h->n64[c] = h->n32[c] = 0;
-    if (h->ntot > 0 && nsub > 0) {
+    if (h->ntile > 0 && nsub > 0) {
         ScreenArgs sa{};
         sa.subs = h->d_subs;
         sa.nsub = nsub;
-        sa.ntot = h->ntot;
+        sa.ntile = h->ntile;
+        sa.tw = h->offs.tw;
         for (int t = 0; t < NPT; ++t) {
             sa.sh[t] = h->d_ash[t];
             sa.schw[t] = h->d_aschw[t];
@@ -1020,21 +1171,20 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
         sa.jonly = jonly;
         sa.f32cut = f32cut;
         sa.cnt = h->d_cnt;
+        sa.tcnt = h->d_tcnt;
+        sa.mask = h->d_mask;
         sa.qbuf = h->d_q;
-        const long long warps = h->ntot / 32;
-        const int blocks = (int)std::min<long long>((warps + 7) / 8, (long long)h->nsm * 64);
-        const size_t cbytes = 2 * (size_t)nsub * sizeof(unsigned long long);
-        HF_CHECK(cudaMemsetAsync(h->d_cnt, 0, cbytes, h->stream));
+        const int blocks = (h->ntile + 7) / 8;
+        HF_CHECK(cudaMemsetAsync(h->d_cnt, 0, 2 * (size_t)nsub * sizeof(unsigned long long), h->stream));
         ++h->launches;
-        k_screen<0><<<blocks, 256, 0, h->stream>>>(sa);  // survivors per sub-class
+        k_screen<<<blocks, 256, 0, h->stream>>>(sa);  // survivor masks and counts
         HF_CHECK(cudaGetLastError());
         ++h->launches;
-        k_offsets<<<NCLS, 32, 0, h->stream>>>(h->offs, h->d_subs, h->d_cnt, h->d_ncls,
-                                              reinterpret_cast<int*>(h->d_ncls + 2 * NCLS));
+        k_offsets<<<NCLS + nsub, OFF_THREADS, 0, h->stream>>>(h->offs, h->d_subs, h->d_cnt, h->d_tcnt, h->d_ncls,
+                                                              reinterpret_cast<int*>(h->d_ncls + 2 * NCLS));
         HF_CHECK(cudaGetLastError());
-        HF_CHECK(cudaMemsetAsync(h->d_cnt, 0, cbytes, h->stream));
         ++h->launches;
-        k_screen<1><<<blocks, 256, 0, h->stream>>>(sa);  // compacted write
+        k_expand<<<blocks, 256, 0, h->stream>>>(sa);  // compacted write
         HF_CHECK(cudaGetLastError());
     }
     {  // the density in shell-pair blocks for the staged scatter
@@ -1298,7 +1448,7 @@ int hfgpu_finalize(hfgpu_handle* h) {
     if (h->gexec) cudaGraphExecDestroy(h->gexec);
     if (h->graph) cudaGraphDestroy(h->graph);
     void* bufs[] = {h->d_shtyp, h->d_aosh, h->d_psoa, h->d_apsoa, h->d_boys, h->d_boysf, h->d_P, h->d_F, h->d_G,
-                    h->d_md, h->d_subs, h->d_q, h->d_cnt, h->d_stats, h->d_scratch, h->d_dscratch,
+                    h->d_md, h->d_subs, h->d_q, h->d_cnt, h->d_mask, h->d_tcnt, h->d_stats, h->d_scratch, h->d_dscratch,
                     h->d_ncls, h->d_Pb, h->d_boff, h->d_aomap, h->d_nfsh};
     for (void* b : bufs)
         if (b) cudaFreeAsync(b, h->stream);
@@ -1640,6 +1790,7 @@ int hfgpu_device_bytes(const hfgpu_handle* h, size_t* bytes) {
     b += h->qcap * sizeof(uint2);                             // quartet lists
     b += h->scratch_doubles * sizeof(double);                 // staged scratch
     b += h->dscratch_doubles * sizeof(double);                // staged diagonal builders' scratch
+    b += h->maskcap * 2 * sizeof(unsigned) + h->tilecap * 2 * sizeof(int);  // screening masks and counts
     b += h->subcap * (sizeof(ScreenSub) + 2 * sizeof(unsigned long long));
     b += (size_t)(BOYS_MMAX + 1) * BOYS_BLK * (sizeof(double) + sizeof(float));
     *bytes = b;
