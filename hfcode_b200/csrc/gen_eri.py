@@ -26,6 +26,7 @@ Run as a script to regenerate ``generated/eri_classes.cuh``.
 """
 from __future__ import annotations
 
+import functools
 import itertools
 import json
 import math
@@ -105,12 +106,72 @@ def fmt_coef(c: float, ft: str) -> str:
     return s if ft == "double" else s + "f"
 
 
+# How the vertical recurrence reduces [e0|f0]^(m): which side first, which
+# axis among those with a non-zero exponent (ties by the axis order).
+VRR_PLANS = [(side, perm, pick) for side in ("bra", "ket", "big", "small")
+             for perm in itertools.permutations(range(3)) for pick in ("max", "min", "first")]
+
+
+def vrr_step(plan, e, f):
+    """(side, axis) by which `plan` reduces (e, f) != (0, 0)."""
+    side, perm, pick = plan
+    se, sf = sum(e), sum(f)
+    if side == "bra":
+        on_bra = se > 0
+    elif side == "ket":
+        on_bra = sf == 0
+    elif side == "big":
+        on_bra = se > 0 and se >= sf
+    else:
+        on_bra = sf == 0 or 0 < se < sf
+    v = e if on_bra else f
+    axes = [k for k in perm if v[k] > 0]
+    if pick == "max":
+        i = max(axes, key=lambda k: v[k])
+    elif pick == "min":
+        i = min(axes, key=lambda k: v[k])
+    else:
+        i = axes[0]
+    return ("bra" if on_bra else "ket"), i
+
+
+@functools.lru_cache(maxsize=None)
+def vrr_plan(targets):
+    """The plan with the fewest FP64 operations (terms and brackets) for the
+    targets [e0|f0]^(0): 10-25% below the better of bra- and ket-first with
+    the largest component for the d-heavy roles."""
+
+    def cost(plan):
+        seen, stack, ops = set(), [(e, f, 0) for e, f in targets], 0
+        while stack:
+            e, f, m = stack.pop()
+            if (e, f, m) in seen or (e == Z3 and f == Z3):
+                continue
+            seen.add((e, f, m))
+            side, i = vrr_step(plan, e, f)
+            v, o = (e, f) if side == "bra" else (f, e)
+            pair = (lambda x, y: (x, y)) if side == "bra" else (lambda x, y: (y, x))
+            v1 = add(v, i, -1)
+            ops += 2
+            stack += [(*pair(v1, o), m), (*pair(v1, o), m + 1)]
+            if v1[i] > 0:
+                v2 = add(v1, i, -1)
+                ops += 2
+                stack += [(*pair(v2, o), m), (*pair(v2, o), m + 1)]
+            if o[i] > 0:
+                ops += 1
+                stack.append((*pair(v1, add(o, i, -1)), m + 1))
+        return ops
+
+    return min((cost(p), n) for n, p in enumerate(VRR_PLANS))
+
+
 class VRR:
     """Obara-Saika vertical recurrence for [e0|f0]^(m), memoised."""
 
-    def __init__(self, em: Emitter, order: str):
+    def __init__(self, em: Emitter, plan):
         self.em = em
-        self.order = order
+        self.plan = plan
         self.nodes: Dict[Tuple, str] = {}
         self.nops = 0
 
@@ -122,13 +183,9 @@ class VRR:
             name = f"B{m}"
             self.nodes[key] = name
             return name
-        if self.order == "bra":
-            side = "bra" if sum(e) > 0 else "ket"
-        else:
-            side = "ket" if sum(f) > 0 else "bra"
+        side, i = vrr_step(self.plan, e, f)
         terms = []
         if side == "bra":
-            i = max(range(3), key=lambda k: (e[k], -k))
             e1 = add(e, i, -1)
             terms.append(f"PA{i}*{self.get(e1, f, m)}")
             terms.append(f"WP{i}*{self.get(e1, f, m + 1)}")
@@ -139,7 +196,6 @@ class VRR:
                 f1 = add(f, i, -1)
                 terms.append(f"h2pq{f[i]}*{self.get(e1, f1, m + 1)}")
         else:
-            i = max(range(3), key=lambda k: (f[k], -k))
             f1 = add(f, i, -1)
             terms.append(f"QC{i}*{self.get(e, f1, m)}")
             terms.append(f"WQ{i}*{self.get(e, f1, m + 1)}")
@@ -272,9 +328,14 @@ class ClassGen:
             s |= self.leaves(c4)
         return s
 
-    def partition(self, acc_max: int, out_max: int):
+    def partition(self, acc_max: int, out_max: int, b_split=None):
         """Greedy split of the outputs (flat order) into roles whose
-        accumulator and output counts fit the register budget."""
+        accumulator and output counts fit the register budget; or, with
+        `b_split`, one role per function of the first shell and block of the
+        second's."""
+        if b_split:
+            return [[n for n, o in enumerate(self.outputs) if o[0] == i and o[1] in blk]
+                    for i in range(self.nf[0]) for blk in b_split]
         groups, cur, cur_acc = [], [], set()
         for n, o in enumerate(self.outputs):
             lv = self.out_leaves(o)
@@ -296,21 +357,23 @@ class ClassGen:
         L = self.L
         cv = (lambda s: s) if dbl else (lambda s: f"(float)({s})")
         targets = sorted({(e, f) for (_, _, e, f) in keys})
-
-        def gen_vrr(order):
-            em = Emitter(ft)
-            v = VRR(em, order)
-            for (e, f) in targets:
-                v.get(e, f, 0)
-            return em, v
-
-        em_b, v_b = gen_vrr("bra")
-        em_k, v_k = gen_vrr("ket")
-        em, vrr = (em_b, v_b) if v_b.nops <= v_k.nops else (em_k, v_k)
         acc = {}
         for key in sorted(keys, key=lambda k: (k[0], k[1], sum(k[2]), k[2], sum(k[3]), k[3])):
             bi, ki, e, f = key
             acc[key] = f"a{bi}{ki}_{''.join(map(str, e))}_{''.join(map(str, f))}"
+        em = Emitter(ft)
+        plan = VRR_PLANS[vrr_plan(tuple(targets))[1]]
+        vrr = VRR(em, plan)
+        # each target is accumulated as soon as it is formed: kept to the end
+        # of the primitive quartet, the targets would all be live at once
+        for (e, f) in targets:
+            src = vrr.get(e, f, 0)
+            for bi in range(len(self.bra_combos)):
+                for ki in range(len(self.ket_combos)):
+                    if (bi, ki, e, f) not in acc:
+                        continue
+                    wexp = ([f"wb{bi}"] if self.bra_combos[bi][2] else []) + ([f"wk{ki}"] if self.ket_combos[ki][2] else [])
+                    em.raw(f"    {acc[bi, ki, e, f]} += {' * '.join(wexp + [src])};")
         out = []
         w = out.append
         w(f"    {ft} " + ", ".join(f"{n} = 0" for n in acc.values()) + ";")
@@ -372,14 +435,6 @@ class ClassGen:
             w(f"            const {ft} wk{ki} = {expr};")
         for line in em.lines:
             w("        " + line)
-        for (bi, ki, e, f), nm in acc.items():
-            src = vrr.nodes[(e, f, 0)]
-            wexp = []
-            if self.bra_combos[bi][2]:
-                wexp.append(f"wb{bi}")
-            if self.ket_combos[ki][2]:
-                wexp.append(f"wk{ki}")
-            w(f"            {nm} += {' * '.join(wexp + [src])};")
         w("        }")
         w("    }")
         # the lanes that share the quartet sum their accumulators (no code
@@ -388,7 +443,7 @@ class ClassGen:
         out += [f"        {nm} = lane_add({nm}, o);" for nm in acc.values()]
         w("    }")
         nbracket = sum(line.count(" - r") for line in em.lines)
-        return out, acc, {"vrr": vrr.nops, "bracket": nbracket, "acc": len(acc), "order": vrr.order}
+        return out, acc, {"vrr": vrr.nops, "bracket": nbracket, "acc": len(acc), "order": plan[0]}
 
     def _hrr_block(self, outs, leaf, ft, store=None):
         """HRR on ket and bra plus the spherical transform for `outs`;
@@ -626,12 +681,15 @@ def acc_groups(g: "ClassGen", group: int = ACC_GROUP):
         "bra": lambda k: (k[0], sum(k[2]), k[2], k[1], sum(k[3]), k[3]),
         "f": lambda k: (sum(k[3]), k[3], k[1], k[0], sum(k[2]), k[2]),
         "e": lambda k: (sum(k[2]), k[2], k[0], k[1], sum(k[3]), k[3]),
+        "fx": lambda k: (k[3], sum(k[2]), k[2], k[0], k[1]),  # by component: groups share a direction
+        "ex": lambda k: (k[2], sum(k[3]), k[3], k[0], k[1]),
     }
+    size = -(-len(keys) // -(-len(keys) // group))  # equal groups of at most `group`
     best = None
     for name, fn in orders.items():
         ks = sorted(keys, key=fn)
-        groups = [ks[i:i + group] for i in range(0, len(ks), group)]
-        cost = sum(g._vrr_block(set(gr))[2]["vrr"] for gr in groups)
+        groups = [ks[i:i + size] for i in range(0, len(ks), size)]
+        cost = sum(vrr_plan(tuple(sorted({(e, f) for (_, _, e, f) in gr})))[0] for gr in groups)
         if best is None or cost < best[0]:
             best = (cost, groups)
     return best[1]
@@ -693,7 +751,7 @@ def class_source(ci: int, bi: int, ki: int):
     g32 = ClassGen(PAIR_TYPES[bi], PAIR_TYPES[ki], "float", suffix="_f32")
     g.flop_model()
     prm = class_params(g.tag)
-    roles = g.partition(prm["acc_max"], prm["out_max"])
+    roles = g.partition(prm["acc_max"], prm["out_max"], prm.get("b_split"))
     funcs, kern = [], []
     reg = []
     NA, NB, NC, ND = g.nf
