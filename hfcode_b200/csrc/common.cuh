@@ -424,33 +424,59 @@ struct StagedArgs {
     UnitList list;
 };
 
-// Unit u of a one-launch stage: false past the end.
-__device__ __forceinline__ bool next_unit(const StagedArgs& a, int u, Unit& w) {
-    if (a.list.subs) {
-        if (!unit_of(a.list, u, w)) return false;
-        // entries of other chunks: not stored (a unit may span two chunks)
-        const long long t = w.t - a.q0;
-        w.store = w.store && t >= 0 && t < a.n;
-        w.t = (int)t;
-        return true;
-    }
-    // diagonal builders: two pairs per warp, their at most 9 x 9 primitive
-    // quartets over 4 x 4 lanes
-    if (2 * u >= a.n) return false;
-    const int lane = threadIdx.x & 31, g = lane & 15, i = 2 * u + (lane >> 4);
-    w.t = i < a.n ? i : a.n - 1;
-    w.q = a.quartets[a.q0 + w.t];
-    w.store = i < a.n && g == 0;
-    w.ls = LaneSplit{g >> 2, 4, g & 3, 4, 16};
-    return true;
-}
-
 // Quartets of this chunk: a.n, or with device-side counts the part of the
 // list left after q0, at most a.n.
 __device__ __forceinline__ int staged_count(const StagedArgs& a) {
     if (!a.ncls) return a.n;
     const long long left = (long long)a.ncls[2 * a.cls + a.prec] - a.q0;
     return (int)(left < 0 ? 0 : left < a.n ? left : a.n);
+}
+
+// Units of the chunk in a one-launch stage, [u0, u1): those of the list that
+// hold its entries (the first and last may reach into a neighbouring chunk,
+// which computes them too), or one per two pairs in the diagonal builders.
+__device__ __forceinline__ void chunk_units(const StagedArgs& a, int& u0, int& u1) {
+    const UnitList& L = a.list;
+    if (!L.subs) {
+        u0 = 0;
+        u1 = (a.n + 1) / 2;
+        return;
+    }
+    const int n = staged_count(a), p = L.prec;
+    u0 = u1 = 0;
+    if (n == 0) return;
+    const long long first = L.coff + (p ? (long long)L.ncls[2 * L.cls] : 0) + a.q0;
+    for (int end = 0; end < 2; ++end) {  // the units of the first and of the last entry
+        const long long at = first + (end ? n - 1 : 0);
+        int lo = L.sub0, hi = L.sub1 - 1;  // last sub-class whose entries start at or before `at`
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (L.subs[mid].off[p] <= at) lo = mid;
+            else hi = mid - 1;
+        }
+        const ScreenSub& S = L.subs[lo];
+        const int u = S.unit[p] + (int)((at - S.off[p]) >> (5 - S.lgb[p] - S.lgk[p]));
+        if (end) u1 = u + 1;
+        else u0 = u;
+    }
+}
+
+// Unit u of a one-launch stage (chunk_units).
+__device__ __forceinline__ void stage_unit(const StagedArgs& a, int u, Unit& w) {
+    if (a.list.subs) {
+        unit_of(a.list, u, w);
+        const long long t = w.t - a.q0;  // entries of other chunks are not stored
+        w.store = w.store && t >= 0 && t < a.n;
+        w.t = (int)t;
+        return;
+    }
+    // diagonal builders: two pairs per warp, their at most 9 x 9 primitive
+    // quartets over 4 x 4 lanes
+    const int lane = threadIdx.x & 31, g = lane & 15, i = 2 * u + (lane >> 4);
+    w.t = i < a.n ? i : a.n - 1;
+    w.q = a.quartets[a.q0 + w.t];
+    w.store = i < a.n && g == 0;
+    w.ls = LaneSplit{g >> 2, 4, g & 3, 4, 16};
 }
 
 // Scratch layout of a chunk.  Each region (accumulators, outputs, role

@@ -721,10 +721,11 @@ def unit_kernel(kname: str, bodies: List[str], minb: int = 2) -> str:
     cases = "\n".join(f"            case {r}: {b}_unit(a, w); break;" for r, b in enumerate(bodies))
     return f"""
 __global__ void __launch_bounds__(RB_THREADS, {minb} * RB_SCALE) {kname}(StagedArgs a) {{
-    if (a.list.subs && staged_count(a) == 0) return;  // a chunk past the end of the list
+    int u0, u1;
+    chunk_units(a, u0, u1);
     Unit w;
-    for (int u = blockIdx.x; next_unit(a, u, w); u += gridDim.x) {{
-        if (!__any_sync(0xffffffffu, w.store)) continue;  // a unit of other chunks
+    for (int u = u0 + blockIdx.x; u < u1; u += gridDim.x) {{
+        stage_unit(a, u, w);
         switch (blockIdx.y) {{
 {cases}
             default: break;

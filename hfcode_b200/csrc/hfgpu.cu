@@ -532,6 +532,8 @@ struct hfgpu_handle {
     uint2* d_diaglist[NPT] = {};   // (i, i) for every pair of a type: staged diagonal builders
     double* d_dscratch = nullptr;  // scratch of the staged diagonal builders
     size_t dstride[NPT] = {};
+    size_t doff[NPT] = {};         // each staged type's part of d_dscratch (all 0 when they share it)
+    bool dshared = false;
     size_t scratch_doubles = 0;
     size_t dscratch_doubles = 0;   // scratch of the staged diagonal builders
     size_t stride[NCLS] = {};      // quartets per chunk of each staged class
@@ -726,9 +728,10 @@ int run_staged_diag(hfgpu_handle* h, int t, int mode, const double* P, double th
         a.prims = h->psoa;
         a.boys = h->d_boys;
         a.boysf = h->d_boysf;
-        a.acc = h->d_dscratch;
-        a.out = h->d_dscratch + (size_t)K.nacc * st;
-        a.mx = h->d_dscratch + (size_t)(K.nacc + K.nout) * st;
+        double* const scratch = h->d_dscratch + h->doff[t];
+        a.acc = scratch;
+        a.out = scratch + (size_t)K.nacc * st;
+        a.mx = scratch + (size_t)(K.nacc + K.nout) * st;
         a.stride = st;
         a.nroles = K.nrole_b;
         a.P = P;
@@ -741,7 +744,7 @@ int run_staged_diag(hfgpu_handle* h, int t, int mode, const double* P, double th
         a.md = md;
         a.nsh = h->nsh;
         // every role of a stage in one launch, two pairs per warp in the
-        // primitive-loop stage (next_unit), then one warp per pair
+        // primitive-loop stage (stage_unit), then one warp per pair
         const int blocks = (m + ND_THREADS - 1) / ND_THREADS, units = (m + 1) / 2;
         if (K.nrole_a > 0) {
             ++h->launches;
@@ -758,37 +761,40 @@ int run_staged_diag(hfgpu_handle* h, int t, int mode, const double* P, double th
     return HFGPU_OK;
 }
 
-// Diagonal builder: the direct pair types on `s_direct`, the staged types
-// (which share one scratch) one after another on `s_staged`.
+// Diagonal builder: the direct pair types on streams[0], the staged types on
+// the next one, or with `spread` each on one of its own (not when they share
+// their scratch).
 int launch_diag(hfgpu_handle* h, int mode, const double* P, double thr, double* G, const double* md,
-                cudaStream_t s_direct, cudaStream_t s_staged) {
+                const cudaStream_t* streams, int ns, bool spread) {
+    int next = 0;
     for (int t = 0; t < NPT; ++t) {
         int n = (int)h->pairs[t].size();
         if (n == 0) continue;
         if (CLASS_KERNELS[class_index(t, t)].mode != 0) {
-            int rc = run_staged_diag(h, t, mode, P, thr, G, md, s_staged);
+            if ((spread && !h->dshared) || next == 0) ++next;
+            int rc = run_staged_diag(h, t, mode, P, thr, G, md, streams[next % ns]);
             if (rc) return rc;
             continue;
         }
         DiagArgs a{h->d_pairs[t], n, h->psoa, h->d_boys, h->d_schw[t], md, h->nsh, P, G, h->d_boff, h->nb, thr};
         ++h->launches;
-        diag_kernel(t, mode)<<<(n + WPB - 1) / WPB, ND_THREADS, 0, s_direct>>>(a);
+        diag_kernel(t, mode)<<<(n + WPB - 1) / WPB, ND_THREADS, 0, streams[0]>>>(a);
         HF_CHECK(cudaGetLastError());
     }
     return HFGPU_OK;
 }
 
-// The diagonal builder on the first two class streams, forked from the
-// handle's stream.  The class streams join back at the end of an
-// off-diagonal build, or here when `join` is set.
+// The diagonal builder on the class streams, forked from the handle's
+// stream: on all of them when nothing else runs (`join`: they join back
+// here), on two beside the screening of an off-diagonal build, which joins
+// them at its end.
 int fork_diag(hfgpu_handle* h, int mode, const double* P, double thr, bool join) {
-    cudaStream_t s0 = h->aux[0], s1 = h->aux[h->nstreams > 1 ? 1 : 0];
+    const int ns = join ? h->nstreams : std::min(2, h->nstreams);
     HF_CHECK(cudaEventRecord(h->fork, h->stream));
-    HF_CHECK(cudaStreamWaitEvent(s0, h->fork, 0));
-    if (s1 != s0) HF_CHECK(cudaStreamWaitEvent(s1, h->fork, 0));
-    const int rc = launch_diag(h, mode, P, thr, h->d_G, h->d_md, s0, s1);
+    for (int k = 0; k < ns; ++k) HF_CHECK(cudaStreamWaitEvent(h->aux[k], h->fork, 0));
+    const int rc = launch_diag(h, mode, P, thr, h->d_G, h->d_md, h->aux, ns, join);
     if (rc || !join) return rc;
-    for (int k = 0; k < (s1 != s0 ? 2 : 1); ++k) {
+    for (int k = 0; k < ns; ++k) {
         HF_CHECK(cudaEventRecord(h->join[k], h->aux[k]));
         HF_CHECK(cudaStreamWaitEvent(h->stream, h->join[k], 0));
     }
@@ -1103,11 +1109,12 @@ int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, d
             // a small list: every role of a stage in one launch, side by side,
             // the primitive-loop stage on the class's work units
             a.list = unit_list(h, c, prec);
-            // a unit holds at least one quartet, so n bounds the units; two
+            // a unit holds at least one quartet, so m bounds the units; two
             // rounds of the eight resident warps per SM in a capture
             const int nr = std::max(na, a.nroles);
             const long long fill = (16LL * h->nsm + nr - 1) / nr;
-            const unsigned units = walk_blocks(capture ? n : h->nunit[2 * c + prec], fill, capture);
+            const long long need = capture ? m : (long long)h->nunit[2 * c + prec] * m / n + 32;  // this chunk's share
+            const unsigned units = walk_blocks(std::min<long long>(m, need), fill, capture);
             const unsigned hblocks = walk_blocks((long long)blocks * RB_SCALE, fill, capture);
             if (na > 0) {
                 ++h->launches;
@@ -1481,7 +1488,7 @@ int hfgpu_finalize(hfgpu_handle* h) {
 static int alloc_diag_scratch(hfgpu_handle* h) {
     if (h->d_dscratch) return HFGPU_OK;
     const size_t budget = h->scratch_budget ? h->scratch_budget / sizeof(double) : scratch_budget_doubles();
-    size_t need = 0;
+    size_t need = 0, sum = 0;
     for (int t = 0; t < NPT; ++t) {
         const ClassKernels& K = CLASS_KERNELS[class_index(t, t)];
         const size_t n = h->pairs[t].size();
@@ -1489,9 +1496,16 @@ static int alloc_diag_scratch(hfgpu_handle* h) {
         const size_t per = (size_t)K.nacc + K.nout + K.nrole_b;
         const size_t st = (std::max<size_t>(std::min<size_t>(n, budget / per), TQ) + TQ - 1) / TQ * TQ;  // whole tiles
         h->dstride[t] = st;
+        h->doff[t] = sum;
         need = std::max(need, st * per);
+        sum += st * per;
     }
     if (!need) return HFGPU_OK;
+    // the staged types run side by side where their parts fit the budget
+    // together, else one after another through one scratch
+    h->dshared = sum > std::max(budget, need);
+    if (h->dshared) std::fill(h->doff, h->doff + NPT, 0);
+    else need = sum;
     const int rc = dalloc(&h->d_dscratch, need, h->stream);
     if (rc == HFGPU_OK) h->dscratch_doubles = need;
     return rc;
@@ -1961,6 +1975,6 @@ extern "C" int hfgpu_fock_build_diag_static(hfgpu_handle* h, double* f_dev, cons
     // G keeps the previous call's sums: clear it first
     HF_CHECK(cudaMemsetAsync(G, 0, (size_t)h->nb * h->nb * sizeof(double), h->stream));
     if ((rc = launch_maxdm(h, p_dev, md))) return rc;
-    if ((rc = launch_diag(h, 1, p_dev, thr, G, md, h->stream, h->stream))) return rc;
+    if ((rc = launch_diag(h, 1, p_dev, thr, G, md, &h->stream, 1, false))) return rc;
     return launch_symm(h, f_dev, G);
 }
