@@ -165,6 +165,135 @@ __global__ void k_sp2_update(double* __restrict__ x, const double* __restrict__ 
     block_add2(d, q, tr_out);
 }
 
+// The whole purification of a small matrix in one launch, by one cluster.
+// Every CTA keeps all of X in shared memory and the cluster's 128 warps share
+// the 8 x 8 tiles of X^2 (the upper ones; X is symmetric) on the FP64 tensor
+// path (mma m8n8k4).  The new tiles go through global memory (two buffers in
+// turn) with one cluster barrier per step.  Each CTA forms the traces, and so
+// the step's choice and the end, from its own copy in the same order, so all
+// CTAs agree without exchanging them.  As a product and an update kernel per
+// step the purification is launches: 28 steps of 12.8 us at nb = 90, where
+// the product itself takes 1.2 us on eight SMs.
+constexpr int SP2C = 8;          // CTAs of the cluster
+constexpr int SP2T = 512;        // threads of a CTA
+constexpr int SP2_MAXN = 160;    // X in shared memory: 160 rows of 164 doubles, 205 KB
+constexpr int SP2_MAXSTEP = 160;
+// leading dimension: 4 modulo 16 doubles, so that the fragment loads (8 rows
+// of 4 doubles) meet no bank conflicts
+__host__ __device__ constexpr int sp2_ld(int n) { return ((n + 7) / 8 * 8 + 15) / 16 * 16 + 4; }
+
+__device__ __forceinline__ void mma_f64(double& d0, double& d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// Sum (OP 0), minimum (1) or maximum (2) of a value over the CTA, the same in every thread.
+template <int OP>
+__device__ __forceinline__ double cta_reduce(double v, double* red) {
+    auto f = [](double a, double b) { return OP == 0 ? a + b : OP == 1 ? fmin(a, b) : fmax(a, b); };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = f(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __syncthreads();  // red may still be read
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = red[0];
+    for (int w = 1; w < SP2T / 32; ++w) v = f(v, red[w]);
+    return v;
+}
+
+// x0, x1: n x n buffers; the projector ends up in x0.  *steps += steps done.
+__global__ void __cluster_dims__(SP2C, 1, 1) __launch_bounds__(SP2T)
+    k_sp2_cluster(const double* __restrict__ f, int n, double nocc, double tol, double* x0, double* x1, int* steps) {
+    extern __shared__ __align__(16) double X[];
+    __shared__ double red[SP2T / 32];
+    const int ld = sp2_ld(n), nt = (n + 7) / 8, np = nt * 8;
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, rank = blockIdx.x;
+    for (int t = tid; t < np * ld; t += SP2T) X[t] = 0.0;
+    __syncthreads();
+    for (int t = tid; t < n * n; t += SP2T) {
+        const int i = t % n, j = t / n;
+        X[j * ld + i] = 0.5 * (f[t] + f[j + (size_t)i * n]);
+    }
+    __syncthreads();
+    // Gershgorin bounds of the symmetric part of f
+    double lo = 1e300, hi = -1e300;
+    for (int i = tid; i < n; i += SP2T) {
+        double r = 0.0;
+        for (int j = 0; j < n; ++j)
+            if (j != i) r += fabs(X[j * ld + i]);
+        lo = fmin(lo, X[i * ld + i] - r);
+        hi = fmax(hi, X[i * ld + i] + r);
+    }
+    lo = cta_reduce<1>(lo, red);
+    hi = cta_reduce<2>(hi, red);
+    __syncthreads();
+    double tr = 0.0, sq = 0.0;
+    for (int t = tid; t < n * n; t += SP2T) {
+        const int i = t % n, j = t / n;
+        const double v = ((i == j ? hi : 0.0) - X[j * ld + i]) / (hi - lo);
+        X[j * ld + i] = v;
+        tr += i == j ? v : 0.0;
+        sq += v * v;
+    }
+    const int g = lane >> 2, q = lane & 3;  // fragment row and column
+    int step = 0, more = -1;                // steps left after convergence
+    while (true) {
+        tr = cta_reduce<0>(tr, red);
+        sq = cta_reduce<0>(sq, red);
+        // tr X - tr X^2 = sum x_k (1 - x_k): zero for a projector.  Two more
+        // steps square what is left on both sides of the gap
+        if (more < 0 && fabs(tr - sq) < tol) more = 2;
+        if (more == 0 || step == SP2_MAXSTEP) break;
+        if (more > 0) --more;
+        const bool square = fabs(sq - nocc) < fabs(2.0 * tr - sq - nocc);
+        double* __restrict__ out = step & 1 ? x0 : x1;
+        // upper tiles (ti <= tj), warp by warp over the cluster
+        for (int t = wp * SP2C + rank; t < nt * (nt + 1) / 2; t += SP2C * (SP2T / 32)) {
+            int tj = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
+            while (tj * (tj + 1) / 2 > t) --tj;
+            while ((tj + 1) * (tj + 2) / 2 <= t) ++tj;
+            const int ti = t - tj * (tj + 1) / 2;
+            const double* a = X + (ti * 8 + g) * ld + q;
+            const double* b = X + (tj * 8 + g) * ld + q;  // X is symmetric: a column is a row
+            double c0 = 0.0, c1 = 0.0, d0 = 0.0, d1 = 0.0;
+            for (int k = 0; k < np; k += 8) {
+                mma_f64(c0, c1, a[k], b[k]);
+                mma_f64(d0, d1, a[k + 4], b[k + 4]);
+            }
+            c0 += d0;
+            c1 += d1;
+            const int i = ti * 8 + g, j = tj * 8 + 2 * q;
+            if (!square) {
+                c0 = 2.0 * X[i * ld + j] - c0;
+                c1 = 2.0 * X[i * ld + j + 1] - c1;
+            }
+            if (i < n && j < n) out[i * n + j] = out[j * n + i] = c0;
+            if (i < n && j + 1 < n) out[i * n + j + 1] = out[(j + 1) * n + i] = c1;
+        }
+        cluster_barrier();
+        tr = sq = 0.0;
+        for (int t = tid; t < n * n; t += SP2T) {
+            const double v = __ldcg(out + t);
+            const int i = t % n, j = t / n;
+            X[j * ld + i] = v;
+            tr += i == j ? v : 0.0;
+            sq += v * v;
+        }
+        __syncthreads();
+        ++step;
+    }
+    // an odd number of steps left the result in x1; x0 is no longer read
+    if (step & 1 || step == 0)
+        for (int t = rank * SP2T + tid; t < n * n; t += SP2C * SP2T) x0[t] = X[(t / n) * ld + t % n];
+    if (rank == 0 && tid == 0) *steps += step;
+}
+
 // The cycle's scalars in one pass: sum P H, sum P F, <R_new, R_j> for the
 // eight history slots, max |R_new| and max |P - Pold|, into out (zeroed).
 struct CycleArgs {
@@ -229,6 +358,7 @@ struct hfgpu_scf {
     double* work = nullptr;     // syevd workspace
     int lwork = 0;
     int* info = nullptr;
+    int* nsteps = nullptr;      // purification steps of the one-launch form, all cycles
     void* blas_ws = nullptr;
     void* arena = nullptr;       // one stream-ordered allocation holding every buffer above
     CycleScalars* sc = nullptr;  // device
@@ -330,6 +460,13 @@ int density_by_purification(hfgpu_scf* s, const double* Fo, double* P) {
     double* bounds = s->aux;
     double* tr = s->aux + 2;  // three slots of (tr X, tr X^2), rotating with the steps
     double* lo = s->aux + 8;
+    if (nb <= SP2_MAXN) {  // one launch; larger matrices fill the GPU with a product per step
+        k_sp2_cluster<<<SP2C, SP2T, (size_t)((nb + 7) / 8 * 8) * sp2_ld(nb) * sizeof(double), s->st>>>(
+            Fo, nb, (double)s->nocc, 1e-11 * std::max(1, s->nocc), X, X2, s->nsteps);
+        SCF_CUDA(cudaGetLastError());
+        SCF_RC(gemm(s, false, false, 1.0, s->X, X, 0.0, X2));
+        return gemm(s, false, true, 2.0, X2, s->X, 0.0, P);
+    }
     k_gershgorin_rows<<<(unsigned)((nb + 7) / 8), 256, 0, s->st>>>(Fo, nb, lo, lo + nb);
     k_gershgorin_bounds<<<1, 1024, 0, s->st>>>(lo, lo + nb, nb, bounds);
     SCF_CUDA(cudaMemsetAsync(tr, 0, 6 * sizeof(double), s->st));
@@ -465,7 +602,7 @@ int create(hfgpu_handle* h, int nocc, double enuc, const double* S, const double
         o_r[k] = take(bytes);
         o_fo[k] = take(bytes);
     }
-    const size_t o_w = take(nb * sizeof(double)), o_info = take(sizeof(int)), o_sc = take(sizeof(CycleScalars));
+    const size_t o_w = take(nb * sizeof(double)), o_info = take(sizeof(int)), o_ns = take(sizeof(int)), o_sc = take(sizeof(CycleScalars));
     const size_t o_aux = take((8 + 2 * (size_t)nb) * sizeof(double)), o_ws = take(ws);
     const size_t o_work = take((size_t)std::max(1, s->lwork) * sizeof(double));
     SCF_CUDA(hfgpu::pool_alloc(&s->arena, off, s->st));
@@ -477,11 +614,16 @@ int create(hfgpu_handle* h, int nocc, double enuc, const double* S, const double
     }
     s->W = (double*)(base + o_w);
     s->info = (int*)(base + o_info);
+    s->nsteps = (int*)(base + o_ns);
     s->sc = (CycleScalars*)(base + o_sc);
     s->aux = (double*)(base + o_aux);
     s->blas_ws = base + o_ws;
     s->work = (double*)(base + o_work);
     s->bytes = off;
+    SCF_CUDA(cudaMemsetAsync(s->nsteps, 0, sizeof(int), s->st));
+    if (nb <= SP2_MAXN)
+        SCF_CUDA(cudaFuncSetAttribute(k_sp2_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      SP2_MAXN * sp2_ld(SP2_MAXN) * (int)sizeof(double)));
     SCF_BLAS(cublasSetWorkspace(s->blas, s->blas_ws, ws));
     SCF_CUDA(cudaMemcpyAsync(s->S, S, bytes, cudaMemcpyHostToDevice, s->st));
     SCF_CUDA(cudaMemcpyAsync(s->H, hcore, bytes, cudaMemcpyHostToDevice, s->st));
@@ -685,6 +827,8 @@ int run(hfgpu_scf* s, const hfgpu_scf_params& prm, hfgpu_scf_result* res) {
         s->ms_build += mb;
         s->ms_density += md;
     }
+    int nsteps = 0;
+    SCF_CUDA(cudaMemcpyAsync(&nsteps, s->nsteps, sizeof(int), cudaMemcpyDeviceToHost, s->st));
     SCF_CUDA(cudaStreamSynchronize(s->st));
     if (res) {
         res->energy = eelec + s->enuc;
@@ -695,7 +839,7 @@ int run(hfgpu_scf* s, const hfgpu_scf_params& prm, hfgpu_scf_result* res) {
         res->converged = converged ? 1 : 0;
         res->full_builds = nfullb;
         res->delta_builds = ndelta;
-        res->sp2_steps = s->sp2_steps;
+        res->sp2_steps = s->sp2_steps + nsteps;
         res->ms_build = s->ms_build;
         res->ms_density = s->ms_density;
     }
