@@ -1316,9 +1316,15 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
     std::vector<HostPair> plist[NPT];
     h->npairs = build_pairs(B, plist, prims, h->refcount);
     for (int t = 0; t < NPT; ++t) h->pairs[t] = std::move(plist[t]);
-    std::vector<double> bt;
-    std::vector<float> btf;
-    build_boys_table(bt, btf);
+    // the same table for every handle: 16200 long-double series, formed once
+    struct BoysTables {
+        std::vector<double> d;
+        std::vector<float> f;
+        BoysTables() { build_boys_table(d, f); }
+    };
+    static const BoysTables tables;
+    const std::vector<double>& bt = tables.d;
+    const std::vector<float>& btf = tables.f;
     cudaError_t ce = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (ce != cudaSuccess) {
         std::string m = std::string("cudaStreamCreate: ") + cudaGetErrorString(ce);
@@ -1369,9 +1375,8 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
         hfgpu_finalize(h);
         return HFGPU_ERR_NOMEM;
     }
-    for (int i = 0; i < 2 * NCLS + 2; ++i) cudaEventCreate(&h->ev[i]);
     cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming);
-    for (int k = 0; k < NSTREAM; ++k) {
+    for (int k = 0; k < h->nstreams; ++k) {
         cudaStreamCreateWithFlags(&h->aux[k], cudaStreamNonBlocking);
         cudaEventCreateWithFlags(&h->join[k], cudaEventDisableTiming);
     }
@@ -1864,6 +1869,8 @@ int hfgpu_launch_count(const hfgpu_handle* h, long long* n) {
 
 int hfgpu_set_timing(hfgpu_handle* h, int on) {
     if (!h) return set_err(HFGPU_ERR_ARG, "null handle");
+    if (on && !h->ev[0])  // the events of the per-class timing
+        for (cudaEvent_t& e : h->ev) HF_CHECK(cudaEventCreate(&e));
     h->timing = on;
     return HFGPU_OK;
 }
