@@ -301,6 +301,44 @@ constexpr int ND_THREADS = 128;
 constexpr int RB_THREADS = HF_RB_THREADS, RB_SCALE = ND_THREADS / RB_THREADS;
 static_assert(RB_THREADS * RB_SCALE == ND_THREADS, "role blocks tile a scratch tile exactly");
 
+// Shared memory of a direct kernel's block, per warp: the output buffer and
+// the block offsets.
+struct NDShared {
+    double tbuf[ND_THREADS / 32][DCH * WST];
+    int tbase[ND_THREADS / 32][NBASE];
+};
+
+// The work units u0, u0 + du, ... of a direct class.
+template <class C, bool F32, typename Real>
+__device__ __forceinline__ void nondiag_units(const UnitList& list, const GPair* __restrict__ bras,
+                                              const GPair* __restrict__ kets, const PrimSoA& prims,
+                                              const Real* __restrict__ boys, const double* __restrict__ Pb,
+                                              double* __restrict__ G, const int* __restrict__ boff, int nsh,
+                                              double thr, bool jonly, ClassStats* stats, int u0, int du,
+                                              NDShared& sh) {
+    constexpr int NA = pt_na(C::BI), NB = pt_nb(C::BI), NC = pt_na(C::KI), ND = pt_nb(C::KI);
+    static_assert(NA * NB * NC * ND == C::NOUT, "class size");
+    unsigned long long nsc = 0, npr = 0;
+    const int wp = threadIdx.x >> 5;
+    Unit w;
+    for (int u = u0 + wp; unit_of(list, u, w); u += du) {
+        const GPair bra = bras[w.q.x];
+        const GPair ket = kets[w.q.y];
+        Real e[C::NOUT];
+        if constexpr (F32) C::eri32(bra, ket, prims, boys, w.ls, e);
+        else C::eri(bra, ket, prims, boys, w.ls, e);
+        Real mx = 0;
+#pragma unroll
+        for (int i = 0; i < C::NOUT; ++i) mx = fmax(mx, fabs(e[i]));
+        const bool act = w.store && !((double)mx < thr);  // fock_build_non_diag.f90:69
+        npr += w.store ? (unsigned long long)(bra.np * ket.np) : 0ull;
+        nsc += act ? 1ull : 0ull;
+        const double s = (bra.sa == bra.sb ? 0.5 : 1.0) * (ket.sa == ket.sb ? 0.5 : 1.0);
+        scatter_quartet<NA, NB, NC, ND>(e, s, bra, ket, act, Pb, boff, nsh, G, jonly, sh.tbuf[wp], sh.tbase[wp]);
+    }
+    if (stats) warp_add_stats(stats, nsc, npr, F32 ? nsc : 0ull);
+}
+
 template <class C, bool F32>
 __global__ void __launch_bounds__(ND_THREADS) k_nondiag(NDArgs a) {
     using Real = typename std::conditional<F32, float, double>::type;
@@ -309,31 +347,36 @@ __global__ void __launch_bounds__(ND_THREADS) k_nondiag(NDArgs a) {
     __shared__ Real sboys[BOYS_BLK];
     if constexpr (F32) stage_boys<C::LL>(sboys, a.boysf);
     else stage_boys<C::LL>(sboys, a.boys);
-    constexpr int NA = pt_na(C::BI), NB = pt_nb(C::BI), NC = pt_na(C::KI), ND = pt_nb(C::KI);
-    static_assert(NA * NB * NC * ND == C::NOUT, "class size");
-    __shared__ double tbuf[ND_THREADS / 32][DCH * WST];
-    __shared__ int tbase[ND_THREADS / 32][NBASE];
-    unsigned long long nsc = 0, npr = 0;
-    const int warps = gridDim.x * (ND_THREADS / 32), wp = threadIdx.x >> 5;
-    Unit w;
-    for (int u = u0 + (threadIdx.x >> 5); unit_of(a.list, u, w); u += warps) {
-        const GPair bra = a.bra[w.q.x];
-        const GPair ket = a.ket[w.q.y];
-        Real e[C::NOUT];
-        if constexpr (F32) C::eri32(bra, ket, a.prims, sboys, w.ls, e);
-        else C::eri(bra, ket, a.prims, sboys, w.ls, e);
-        Real mx = 0;
-#pragma unroll
-        for (int i = 0; i < C::NOUT; ++i) mx = fmax(mx, fabs(e[i]));
-        const bool act = w.store && !((double)mx < a.thr);  // fock_build_non_diag.f90:69
-        npr += w.store ? (unsigned long long)(bra.np * ket.np) : 0ull;
-        nsc += act ? 1ull : 0ull;
-        const double s = (bra.sa == bra.sb ? 0.5 : 1.0) * (ket.sa == ket.sb ? 0.5 : 1.0);
-        scatter_quartet<NA, NB, NC, ND>(e, s, bra, ket, act, a.Pb, a.boff, a.nsh, a.G, a.jonly != 0, tbuf[wp],
-                                        tbase[wp]);
-    }
-    if (a.stats) warp_add_stats(a.stats, nsc, npr, F32 ? nsc : 0ull);
+    __shared__ NDShared sh;
+    nondiag_units<C, F32, Real>(a.list, a.bra, a.ket, a.prims, sboys, a.Pb, a.G, a.boff, a.nsh, a.thr, a.jonly != 0,
+                                a.stats, u0, gridDim.x * (ND_THREADS / 32), sh);
 }
+
+// Every direct class of a small build in one launch: the blocks are dealt out
+// to the lists in turn.  One launch per class leaves a dozen kernels of
+// 20-35 us, each too short to fill the GPU, on the class streams.  The Boys
+// tables are read through L1 here: most blocks do one unit per warp.
+constexpr int MAXDIRECT = 64;
+struct NDItem {
+    UnitList list;
+    const GPair* bra;
+    const GPair* ket;
+    ClassStats* stats;
+    int block0, blocks;  // this list's blocks of the grid
+};
+struct NDAllArgs {
+    int nitem;
+    PrimSoA prims;
+    const double* boys;
+    const float* boysf;
+    const double* Pb;
+    double* G;
+    const int* boff;
+    int nsh;
+    double thr;
+    int jonly;
+    NDItem item[MAXDIRECT];
+};
 
 struct DiagArgs {
     const GPair* pairs;
@@ -773,6 +816,7 @@ __global__ void __launch_bounds__(ND_THREADS) k_scatter_diag(StagedArgs a) {
 }
 
 typedef void (*NDKernel)(NDArgs);
+typedef void (*NDAllKernel)(const NDAllArgs);
 typedef void (*DiagKernel)(DiagArgs);
 typedef void (*StagedKernel)(StagedArgs);
 constexpr int MAXR = 64;

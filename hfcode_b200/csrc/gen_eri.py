@@ -979,6 +979,49 @@ void register_class_{ci}(ClassKernels* k) {{
 """
 
 
+def write_if_changed(path: str, text: str):
+    if not os.path.exists(path) or open(path).read() != text:
+        with open(path, "w") as fh:
+            fh.write(text)
+
+
+def direct_all(outdir: str, infos: dict):
+    """The one-launch kernels over every direct class, one per precision."""
+    out = []
+    for f32 in (False, True):
+        real, name = ("float", "k_direct_all32") if f32 else ("double", "k_direct_all64")
+        direct = [(ci, i) for ci, i in infos.items() if i["mode"] == "direct"]
+        lines = ["// GENERATED by gen_eri.py -- do not edit.",
+                 f"// The direct classes of a small build in one launch ({'FP32' if f32 else 'FP64'}).",
+                 '#include "../common.cuh"']
+        lines += [f'#include "cls_{ci:02d}_{i["tag"]}.cuh"' for ci, i in direct]
+        lines += ["", "namespace hfgpu {"]
+        lines += [f"HF_CLASS_TRAITS({ci}, {class_list()[ci][0]}, {class_list()[ci][1]}, {i['tag']}, {i['nout']}, {i['L']})"
+                  for ci, i in direct]
+        lines += [f"__global__ void __launch_bounds__(ND_THREADS, 4) {name}(const __grid_constant__ NDAllArgs a) {{",
+                  "    int k = 0;",
+                  "    while (k + 1 < a.nitem && a.item[k + 1].block0 <= (int)blockIdx.x) ++k;",
+                  "    const NDItem& it = a.item[k];",
+                  "    const int u0 = ((int)blockIdx.x - it.block0) * (ND_THREADS / 32), du = it.blocks * (ND_THREADS / 32);",
+                  "    if (u0 >= it.list.nunit[2 * it.list.cls + it.list.prec]) return;",
+                  "    __shared__ NDShared sh;",
+                  "    switch (it.list.cls) {"]
+        for ci, i in direct:
+            tab = "a.boysf" if f32 else "a.boys"
+            lines.append(f"        case {ci}:")
+            lines.append(f"            nondiag_units<Cls_{i['tag']}, {'true' if f32 else 'false'}, {real}>(it.list, it.bra, it.ket, "
+                         f"a.prims, {tab} + (size_t){i['L']} * BOYS_BLK, a.Pb, a.G, a.boff, a.nsh, a.thr, a.jonly != 0, "
+                         f"it.stats, u0, du, sh);")
+            lines.append("            break;")
+        lines += ["        default: break;", "    }", "}",
+                  f"NDAllKernel direct_all{'32' if f32 else '64'}() {{ return {name}; }}", "}  // namespace hfgpu", ""]
+        path = os.path.join(outdir, f"direct_all{'32' if f32 else '64'}.cu")
+        write_if_changed(path, "\n".join(lines))
+        out.append(path)
+    assert len(direct) <= 64
+    return out
+
+
 def main(outdir: str):
     os.makedirs(outdir, exist_ok=True)
     names = []
@@ -992,6 +1035,7 @@ def main(outdir: str):
                 with open(base + ext, "w") as fh:
                     fh.write(text)
         names.append(base + ".cu")
+    names += direct_all(outdir, flops)
     # host dispatch used by the host-compiled check of the generated code
     lines = ["// GENERATED by gen_eri.py -- host dispatch of the class functions (tests only).", ""]
     for ci, info in flops.items():

@@ -47,6 +47,8 @@ namespace hfgpu {
 #define HF_DECL_REG(ci) void register_class_##ci(ClassKernels* k);
 HF_FOR_EACH_CLASS(HF_DECL_REG)
 #undef HF_DECL_REG
+NDAllKernel direct_all64();
+NDAllKernel direct_all32();
 static_assert(HF_NPT == NPT && HF_NCLS == NCLS, "generated class table out of date");
 }  // namespace hfgpu
 
@@ -559,6 +561,7 @@ struct hfgpu_handle {
     OffsetArgs offs{};                  // sub-class ranges / list regions per class
     // [2 * NCLS] surviving quartets (FP64, FP32) per class, then as ints the work units
     unsigned long long* d_ncls = nullptr;
+    long long direct_blocks = 0;        // direct classes of up to this many blocks together run in one launch
     long long warp_scatter = 0;         // chunks up to this many quartets use the one-warp-per-quartet scatter
     double* d_Pb = nullptr;             // density in shell-pair blocks (nb x nb)
     int* d_boff = nullptr;              // block offsets (nsh x nsh)
@@ -1068,6 +1071,11 @@ unsigned walk_blocks(long long need, long long fill, bool capture) {
     return (unsigned)std::max<long long>(1, capture ? std::min(need, fill) : need);
 }
 
+// Blocks of a direct class's list of (at most) n quartets.
+long long direct_need(const hfgpu_handle* h, int c, int prec, long long n, bool capture) {
+    return walk_blocks(((capture ? n : h->nunit[2 * c + prec]) + WPB - 1) / WPB, 8LL * h->nsm, capture);
+}
+
 // Staged class: chunks of the quartet list through the accumulator roles
 // (mode 2), the output roles and the scatter kernel.
 int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, double thr, int jonly,
@@ -1231,7 +1239,46 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
         for (int k = 0; k < h->nstreams; ++k) HF_CHECK(cudaStreamWaitEvent(h->aux[k], h->fork, 0));
     }
     double load[NSTREAM] = {};
+    // the direct classes of a small build side by side in one launch per precision
+    long long direct_blocks = 0;
+    for (const Item& it : items)
+        if (CLASS_KERNELS[it.c].mode == 0) direct_blocks += direct_need(h, it.c, it.prec, it.n, capture);
+    const bool one_launch = multi && direct_blocks <= h->direct_blocks;
+    for (int prec = 0; one_launch && prec < 2; ++prec) {
+        NDAllArgs a{};
+        int blocks = 0;
+        double w = 0.0;
+        for (const Item& it : items) {
+            const ClassKernels& K = CLASS_KERNELS[it.c];
+            if (K.mode != 0 || it.prec != prec) continue;
+            NDItem& d = a.item[a.nitem++];
+            d.list = unit_list(h, it.c, prec);
+            d.bra = h->d_apairs[K.bi];
+            d.ket = h->d_apairs[K.ki];
+            d.stats = h->d_stats + it.c;
+            d.block0 = blocks;
+            d.blocks = (int)direct_need(h, it.c, prec, it.n, capture);
+            blocks += d.blocks;
+            w += it.w;
+        }
+        if (!a.nitem) continue;
+        a.prims = h->apsoa;
+        a.boys = h->d_boys;
+        a.boysf = h->d_boysf;
+        a.Pb = h->d_Pb;
+        a.G = h->d_G;
+        a.boff = h->d_boff;
+        a.nsh = h->nsh;
+        a.thr = thr;
+        a.jonly = jonly;
+        const int k = h->nstreams - 1 - prec % h->nstreams;  // first on its stream: it takes longest
+        load[k] += w;
+        ++h->launches;
+        (prec ? direct_all32() : direct_all64())<<<blocks, ND_THREADS, 0, h->aux[k]>>>(a);
+        HF_CHECK(cudaGetLastError());
+    }
     for (const Item& it : items) {
+        if (one_launch && CLASS_KERNELS[it.c].mode == 0) continue;
         const int c = it.c, prec = it.prec;
         const long long n = it.n;
         const ClassKernels& K = CLASS_KERNELS[c];
@@ -1258,8 +1305,7 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
             a.thr = thr;
             a.jonly = jonly;
             a.stats = h->d_stats + c;
-            const unsigned blocks =
-                walk_blocks(((capture ? n : h->nunit[2 * c + prec]) + WPB - 1) / WPB, 8LL * h->nsm, capture);
+            const unsigned blocks = (unsigned)direct_need(h, c, prec, n, capture);
             ++h->launches;
             (prec ? K.nd32 : K.nd64)<<<blocks, ND_THREADS, 0, st>>>(a);
             HF_CHECK(cudaGetLastError());
@@ -1342,6 +1388,8 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
         h->merge_blocks = 8LL * h->nsm;
         if (const char* e = getenv("HFGPU_MERGE_BLOCKS")) h->merge_blocks = atoll(e);
         h->warp_scatter = 16LL * h->nsm;
+        h->direct_blocks = 64LL * h->nsm;
+        if (const char* e = getenv("HFGPU_DIRECT")) h->direct_blocks = atoll(e);
         if (const char* e = getenv("HFGPU_WARP_SCATTER")) h->warp_scatter = atoll(e);
         if (const char* e = getenv("HFGPU_STREAMS")) h->nstreams = std::max(1, std::min(NSTREAM, atoi(e)));
     }
