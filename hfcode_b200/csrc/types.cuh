@@ -13,9 +13,13 @@ constexpr int NPT = 10;                 // GPU pair types SS LS LL DS DL DD PS L
 constexpr int NCLS = 55;                // quartet classes over the pair types (21 without pure p)
 constexpr int BOYS_NPT = 225;           // grid T_j = j/8, j = 0..224 (T <= 28)
 constexpr int BOYS_K = 8;               // Taylor terms per grid point
-// one block per order M: BOYS_NPT x BOYS_K Taylor coefficients, then the
-// BOYS_NPT values exp(-T_j) used by the downward recursion
-constexpr int BOYS_BLK = BOYS_NPT * (BOYS_K + 1);
+// one block per order M: for each grid point the BOYS_K Taylor coefficients
+// and then exp(-T_j), used by the downward recursion.  The odd row length
+// keeps the lanes of a warp, each at its own grid point, off one another's
+// banks where the table is in shared memory: with rows of eight doubles every
+// load met two banks' worth of rows, a 16-way conflict.
+constexpr int BOYS_ROW = BOYS_K + 1;
+constexpr int BOYS_BLK = BOYS_NPT * BOYS_ROW;
 constexpr int BOYS_MMAX = 8;            // highest order used: (dd|dd)
 
 // Primitive pair (one surviving primitive product of a shell pair): exponent
@@ -124,7 +128,7 @@ __device__ __forceinline__ void boys_eval(double T, const double* __restrict__ t
     } else {
         const int j = __double2int_rn(T * 8.0);
         const double x = T - 0.125 * j;
-        const double* c = tab + j * BOYS_K;
+        const double* c = tab + j * BOYS_ROW;
         double f = c[BOYS_K - 1];
 #pragma unroll
         for (int k = BOYS_K - 2; k >= 0; --k) f = fma(f, x, c[k]);
@@ -143,7 +147,7 @@ __device__ __forceinline__ void boys_eval(double T, const double* __restrict__ t
             ex = fma(ex, -x, 0.5);
             ex = fma(ex, -x, 1.0);
             ex = fma(ex, -x, 1.0);
-            const double e = tab[BOYS_NPT * BOYS_K + j] * ex;
+            const double e = c[BOYS_K] * ex;
             const double t2 = T + T;
 #pragma unroll
             for (int m = M - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], e) * (1.0 / (2 * m + 1));
@@ -162,7 +166,7 @@ __device__ __forceinline__ void boys_eval(float T, const float* __restrict__ tab
     } else {
         const int j = __float2int_rn(T * 8.0f);
         const float x = T - 0.125f * j;
-        const float* c = tab + j * BOYS_K;
+        const float* c = tab + j * BOYS_ROW;
         float f = c[5];
 #pragma unroll
         for (int k = 4; k >= 0; --k) f = fmaf(f, x, c[k]);
