@@ -220,7 +220,7 @@ __device__ __forceinline__ void advance(const ScreenSub& S, int& i, int& j) {
 // and their counts.  Bound by the five density gathers of a candidate (L1);
 // one search and one division per tile instead of one per 32 candidates, and
 // a second pass that expands the masks instead of screening again, took the
-// two passes from 1.71 + 1.98 ms to 0.95 + 0.45 ms on C60 (4.2e8 candidates).
+// two passes from 1.71 + 1.98 ms to 0.85 + 0.19 ms on C60 (4.2e8 candidates).
 __global__ void __launch_bounds__(256) k_screen(ScreenArgs a) {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -822,8 +822,13 @@ size_t scratch_budget_doubles() {
 }
 
 // Fewest primitive quartets per lane of a work unit: below these the sum of
-// the accumulators over the lanes costs more than the shorter loops save.
-constexpr int LMIN_DIRECT = 6, LMIN_STAGED = 4;
+// the accumulators over the lanes, and the recurrences past the loops that
+// every lane then repeats, cost more than the shorter loops save.  Benzene on
+// host arrays (direct / staged): 787 us at 3 / 2, 733 at 6 / 4, 684 at 12 / 8,
+// 654 at 24 / 8; (H2O)12: 773, 742, 694, 670 us; eight molecules in one batch
+// launch: 7.78, 7.50, 7.24, 7.02 ms (the last with half the threads in
+// `fill`, which alone gave 7.36).
+constexpr int LMIN_DIRECT = 24, LMIN_STAGED = 8;
 
 // Schwarz ordering (index_sort + find_threshold) and the active pair arrays.
 int build_active(hfgpu_handle* h) {
@@ -964,13 +969,13 @@ int build_active(hfgpu_handle* h) {
         h->offs.coff[c] = qoff;
         qoff += ccap;
         h->offs.csub[c + 1] = (int)h->hsubs.size();
-        // threads that fill the GPU: 32 warps per SM of a direct kernel, 8 of
+        // threads that fill the GPU: 16 warps per SM of a direct kernel, 8 of
         // the 255-register role kernels, whose roles run side by side
         const ClassKernels& K = CLASS_KERNELS[c];
         for (int p = 0; p < 2; ++p) {
             const int roles = K.mode == 0 ? 1 : K.mode == 1 ? (p ? K.nrole_b32 : K.nrole_b)
                                                             : (p ? K.nrole_a32 : K.nrole_a);
-            h->offs.fill[c][p] = (float)h->nsm * (K.mode == 0 ? 1024.f : 256.f) / (float)roles;
+            h->offs.fill[c][p] = (float)h->nsm * (K.mode == 0 ? 512.f : 256.f) / (float)roles;
         }
         h->offs.lmin[c] = K.mode == 0 ? LMIN_DIRECT : LMIN_STAGED;
     }
