@@ -10,13 +10,14 @@
 //                  skip |e|>1e-10) and fock_build_diag.f90 (M=1: density
 //                  screen schw^2*max(D_ab,D_aa/4,D_bb/4) < thr)
 //   k_screen       the per-quartet screen of fock_build_non_diag.f90:63-67
-//                  (schw_ab*schw_cd*max(Dcoul,Dexch/4) < thr), evaluated for
-//                  every candidate pair of active shell pairs and compacted
-//                  into per-class quartet lists with warp ballots
-//   k_nondiag<C>   one thread per screened shell quartet: contracted (ab|cd)
-//                  from the generated class function, the post-screen
-//                  max|e| < thr (fock_build_non_diag.f90:69), then the J/K
-//                  scatter with FP64 atomics into a one-triangle buffer G
+//                  (schw_ab*schw_cd*max(Dcoul,Dexch/4) < thr), evaluated once
+//                  for every candidate pair of active shell pairs, as bit masks;
+//                  k_expand turns them into per-class quartet lists in order
+//   k_offsets      list offsets and work units: how many lanes share a quartet
+//   k_nondiag<C>   the work units of a direct class: contracted (ab|cd) from
+//                  the generated class function, the post-screen max|e| < thr
+//                  (fock_build_non_diag.f90:69), then the J/K scatter with FP64
+//                  atomics into a one-triangle buffer G in shell-pair blocks
 //   k_symm         F += G + G^T (the reference writes both triangles)
 //
 // The reference's per-case scatter branches (aa|aa), (aa|bc), (ab|cd), ...
