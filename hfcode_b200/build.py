@@ -52,7 +52,7 @@ def build(jobs: int = 0, verbose: bool = True) -> str:
     gen_srcs = gen_eri.main(os.path.join(CSRC, "generated"))
     os.makedirs(BUILD, exist_ok=True)
     common = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "types.cuh"), os.path.join(CSRC, "pairs.hpp"),
-              os.path.join(CSRC, "scatter.cuh"),
+              os.path.join(CSRC, "scatter.cuh"), os.path.join(CSRC, "lists.cuh"),
               os.path.join(HERE, "..", "include", "hfgpu.h"),
               os.path.join(HERE, "..", "include", "hfgpu_basis.h"),
               os.path.join(HERE, "..", "include", "hfgpu_ingest.h"),

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "types.cuh"
+#include "lists.cuh"
 #include "scatter.cuh"
 
 #include <cstdint>
@@ -185,69 +186,11 @@ struct ClassStats {
     unsigned long long scattered, prim, fp32;
 };
 
-// One screening sub-class: the candidates of quartet class `cls` whose bra
-// pairs come from one primitive-count group of the active bra list and ket
-// pairs from one group of the ket list, so that every quartet in the
-// compacted sub-list runs its primitive loops with the same trip counts.
-struct ScreenSub {
-    long long ncand;   // candidates
-    int tile0;         // first screening tile
-    int cls;
-    int same;          // one group against itself: pairs i > j only
-    int b0, nbra;      // bra range in the active list
-    int k0, nket;      // ket range
-    int npb, npk;      // primitives of the bra and ket pairs
-    // filled on the device by k_offsets, FP64 and FP32 entries:
-    long long off[2];  // write offsets (second pass)
-    int unit[2];       // first work unit within the class's list (see Unit)
-    int lgb[2], lgk[2];  // log2 of the lanes over the bra and ket primitives
-};
-
-// Work unit of a class list: one warp's share, 32 / 2^(lgb + lgk) quartets of
-// one sub-class, each spread over 2^(lgb + lgk) lanes that split its
-// primitive loops.  A quartet of two six-fold contracted s pairs runs 1296
-// primitive quartets: one thread per quartet made that one thread's serial
-// chain the time of the whole kernel for a small molecule (benzene SS|SS:
-// 255 us at 66 blocks).
-struct Unit {
-    int t;             // entry within the class's list of this precision
-    bool store;        // this lane writes the quartet's results
-    uint2 q;           // (bra, ket)
-    LaneSplit ls;
-};
-
-struct UnitList {
-    const ScreenSub* subs;             // the sub-class table
-    const unsigned long long* cnt;     // [2 * nsub] entries per sub-class (FP64, FP32)
-    const unsigned long long* ncls;    // [2 * NCLS] entries per class
-    const int* nunit;                  // [2 * NCLS] work units per class
-    int sub0, sub1;                    // sub-classes of this class
-    long long coff;                    // first entry of this class in the quartet buffer
-    const uint2* quartets;             // the whole quartet buffer
-    int cls, prec;
-};
-
-// Unit u of the list: false past the end.  The lanes without a quartet (the
-// tail of a sub-class) repeat the sub-class's last one and do not store.
+// Unit u of the list: false past the end (see unit_place).
 __device__ __forceinline__ bool unit_of(const UnitList& L, int u, Unit& w) {
-    const int p = L.prec;
-    if (u >= L.nunit[2 * L.cls + p]) return false;
-    int lo = L.sub0, hi = L.sub1 - 1;  // last sub-class whose first unit is <= u
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (L.subs[mid].unit[p] <= u) lo = mid;
-        else hi = mid - 1;
-    }
-    const ScreenSub& S = L.subs[lo];
-    const int lgb = S.lgb[p], lgk = S.lgk[p], lg = lgb + lgk, lane = threadIdx.x & 31;
-    const int n = (int)L.cnt[2 * lo + p];
-    const int i = ((u - S.unit[p]) << (5 - lg)) + (lane >> lg);
-    const int g = lane & ((1 << lg) - 1);
-    const long long at = S.off[p] + (i < n ? i : n - 1);
+    const long long at = unit_place(L, u, threadIdx.x & 31, w);
+    if (at < 0) return false;
     w.q = L.quartets[at];
-    w.t = (int)(at - L.coff - (p ? (long long)L.ncls[2 * L.cls] : 0));
-    w.store = i < n && g == 0;
-    w.ls = LaneSplit{g >> lgk, 1 << lgb, g & ((1 << lgk) - 1), 1 << lgk, 1 << lg};
     return true;
 }
 
@@ -485,32 +428,17 @@ __device__ __forceinline__ void chunk_units(const StagedArgs& a, int& u0, int& u
         u1 = (a.n + 1) / 2;
         return;
     }
-    const int n = staged_count(a), p = L.prec;
+    const int n = staged_count(a);
     u0 = u1 = 0;
-    if (n == 0) return;
-    const long long first = L.coff + (p ? (long long)L.ncls[2 * L.cls] : 0) + a.q0;
-    for (int end = 0; end < 2; ++end) {  // the units of the first and of the last entry
-        const long long at = first + (end ? n - 1 : 0);
-        int lo = L.sub0, hi = L.sub1 - 1;  // last sub-class whose entries start at or before `at`
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (L.subs[mid].off[p] <= at) lo = mid;
-            else hi = mid - 1;
-        }
-        const ScreenSub& S = L.subs[lo];
-        const int u = S.unit[p] + (int)((at - S.off[p]) >> (5 - S.lgb[p] - S.lgk[p]));
-        if (end) u1 = u + 1;
-        else u0 = u;
-    }
+    if (n > 0) units_of(L, list_start(L) + a.q0, n, u0, u1);
 }
 
 // Unit u of a one-launch stage (chunk_units).
 __device__ __forceinline__ void stage_unit(const StagedArgs& a, int u, Unit& w) {
     if (a.list.subs) {
         unit_of(a.list, u, w);
-        const long long t = w.t - a.q0;  // entries of other chunks are not stored
-        w.store = w.store && t >= 0 && t < a.n;
-        w.t = (int)t;
+        w.t -= a.q0;  // entries of other chunks are not stored
+        w.store = w.store && w.t >= 0 && w.t < a.n;
         return;
     }
     // diagonal builders: two pairs per warp, their at most 9 x 9 primitive

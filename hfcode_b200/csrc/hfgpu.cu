@@ -169,7 +169,7 @@ struct ScreenArgs {
     int jonly;
     double f32cut;
     unsigned long long* cnt;  // [2*nsub] survivors per sub-class (FP64, FP32)
-    int* tcnt;                // [2*ntile] survivors per tile; after k_offsets the entries before it in its sub-class
+    TileEntries* tcnt;        // [ntile] survivors per tile; after k_offsets the entries before it in its sub-class
     unsigned* mask;           // [tw] survivors per tile, then (f32cut > 0) the FP32 ones of every tile
     uint2* qbuf;
 };
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) k_screen(ScreenArgs a) {
         n64 += __shfl_xor_sync(0xffffffffu, n64, o);
         n32 += __shfl_xor_sync(0xffffffffu, n32, o);
     }
-    if (lane < 2) a.tcnt[2 * t + lane] = lane ? n32 : n64;
+    if (lane == 0) a.tcnt[t] = TileEntries{n64, n32};
     if (lane == 0 && n64) atomicAdd(&a.cnt[2 * c], (unsigned long long)n64);
     if (lane == 1 && n32) atomicAdd(&a.cnt[2 * c + 1], (unsigned long long)n32);
 }
@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(256) k_expand(ScreenArgs a) {
     const int c = tile_sub(a, t);
     const ScreenSub S = a.subs[c];
     const long long u0 = (long long)(t - S.tile0) * (32 * a.tw);
-    long long o64 = S.off[0] + a.tcnt[2 * t], o32 = S.off[1] + a.tcnt[2 * t + 1];
+    const TileEntries before = a.tcnt[t];
+    long long o64 = S.off[0] + before.n64, o32 = S.off[1] + before.n32;
     int i, j;
     candidate(S, u0 + lane, i, j);
     const int words = (int)((min((long long)(32 * a.tw), S.ncand - u0) + 31) >> 5);
@@ -329,23 +330,6 @@ struct OffsetArgs {
     int tw;                  // words per screening tile
 };
 
-// Fewest lanes (lgb + lgk) over npb x npk primitives with at most `most`
-// primitive quartets per lane, and their best split over bra and ket.
-__device__ __forceinline__ void pick_lanes(int npb, int npk, int most, int& lgb, int& lgk) {
-    lgb = lgk = 0;
-    int best = npb * npk;
-    for (int lg = 1; lg <= 5 && best > most; ++lg)
-        for (int k = 0; k <= lg; ++k) {
-            const int b = lg - k;
-            const int c = ((npb + (1 << b) - 1) >> b) * ((npk + (1 << k) - 1) >> k);
-            if (c < best) {
-                best = c;
-                lgb = b;
-                lgk = k;
-            }
-        }
-}
-
 __device__ __forceinline__ long long warp_scan(long long v, int lane) {  // inclusive
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -353,34 +337,6 @@ __device__ __forceinline__ long long warp_scan(long long v, int lane) {  // incl
         if (lane >= o) v += x;
     }
     return v;
-}
-
-// Exclusive sums of a sub-class's tile counts (FP64 and FP32), by one block.
-constexpr int OFF_THREADS = 128;
-__device__ __forceinline__ void scan_tiles(const ScreenSub& S, int tw, int* __restrict__ tcnt) {
-    __shared__ int part[OFF_THREADS / 32][2];
-    const int nt = (int)((S.ncand + 32 * tw - 1) / (32 * tw)), lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    int2* __restrict__ t = reinterpret_cast<int2*>(tcnt) + S.tile0;
-    int2 run = make_int2(0, 0);
-    for (int k0 = 0; k0 < nt; k0 += OFF_THREADS) {
-        const int k = k0 + (int)threadIdx.x;
-        const int2 v = k < nt ? t[k] : make_int2(0, 0);
-        int2 s = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int x = __shfl_up_sync(0xffffffffu, s.x, o), y = __shfl_up_sync(0xffffffffu, s.y, o);
-            if (lane >= o) s.x += x, s.y += y;
-        }
-        if (lane == 31) part[wp][0] = s.x, part[wp][1] = s.y;
-        __syncthreads();
-        int2 before = run;
-        for (int q = 0; q < OFF_THREADS / 32; ++q) {
-            if (q < wp) before.x += part[q][0], before.y += part[q][1];
-            run.x += part[q][0], run.y += part[q][1];
-        }
-        if (k < nt) t[k] = make_int2(before.x + s.x - v.x, before.y + s.y - v.y);
-        __syncthreads();
-    }
 }
 
 // Write offsets of the compacted lists from the screen's counts, on the device
@@ -395,11 +351,13 @@ __device__ __forceinline__ void scan_tiles(const ScreenSub& S, int tw, int* __re
 // entries before the tile.
 __global__ void __launch_bounds__(OFF_THREADS) k_offsets(OffsetArgs o, ScreenSub* __restrict__ subs,
                                                          const unsigned long long* __restrict__ cnt,
-                                                         int* __restrict__ tcnt, unsigned long long* __restrict__ ncls,
+                                                         TileEntries* __restrict__ tcnt,
+                                                         unsigned long long* __restrict__ ncls,
                                                          int* __restrict__ nunit) {
     const int c = blockIdx.x, lane = threadIdx.x;
     if (c >= NCLS) {
-        scan_tiles(subs[c - NCLS], o.tw, tcnt);
+        const ScreenSub& S = subs[c - NCLS];
+        scan_tiles(tcnt + S.tile0, (int)((S.ncand + 32 * o.tw - 1) / (32 * o.tw)));
         return;
     }
     if (lane >= 32) return;
@@ -545,7 +503,7 @@ struct hfgpu_handle {
     size_t naprims = 0;            // primitive pairs of the active lists
     unsigned long long* d_cnt = nullptr;
     unsigned* d_mask = nullptr;    // survivor masks of the screening tiles (all, then the FP32 ones)
-    int* d_tcnt = nullptr;         // survivors per tile (FP64, FP32)
+    TileEntries* d_tcnt = nullptr;  // survivors per tile
     size_t tilecap = 0, maskcap = 0;  // tiles and mask words the two hold
     ClassStats* d_stats = nullptr;
     // last build statistics
@@ -998,7 +956,7 @@ int build_active(hfgpu_handle* h) {
         dfree(h->d_tcnt, h->stream);
         h->tilecap = h->maskcap = 0;
         int rc = dalloc(&h->d_mask, 2 * (size_t)tiles * tw, h->stream);
-        if (rc == HFGPU_OK) rc = dalloc(&h->d_tcnt, 2 * (size_t)tiles, h->stream);
+        if (rc == HFGPU_OK) rc = dalloc(&h->d_tcnt, (size_t)tiles, h->stream);
         if (rc) return rc;
         h->tilecap = (size_t)tiles;
         h->maskcap = (size_t)tiles * tw;
@@ -1863,7 +1821,7 @@ int hfgpu_device_bytes(const hfgpu_handle* h, size_t* bytes) {
     b += h->qcap * sizeof(uint2);                             // quartet lists
     b += h->scratch_doubles * sizeof(double);                 // staged scratch
     b += h->dscratch_doubles * sizeof(double);                // staged diagonal builders' scratch
-    b += h->maskcap * 2 * sizeof(unsigned) + h->tilecap * 2 * sizeof(int);  // screening masks and counts
+    b += h->maskcap * 2 * sizeof(unsigned) + h->tilecap * sizeof(TileEntries);  // screening masks and counts
     b += h->subcap * (sizeof(ScreenSub) + 2 * sizeof(unsigned long long));
     b += (size_t)(BOYS_MMAX + 1) * BOYS_BLK * (sizeof(double) + sizeof(float));
     *bytes = b;
