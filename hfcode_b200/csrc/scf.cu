@@ -125,6 +125,10 @@ __device__ __forceinline__ void block_add2(double a, double b, double* acc) {
     }
 }
 
+// Width of the spectrum's bounds; 1 for a multiple of the identity, whose
+// start is then X = 0: no projector of the wanted rank, and reported as such.
+__device__ __forceinline__ double sp2_range(double lo, double hi) { return hi > lo ? hi - lo : 1.0; }
+
 // X = (hi I - F) / (hi - lo): the start of the purification, spectrum in [0, 1]
 // with the occupied orbitals (lowest energies) nearest 1.  Adds tr X and
 // ||X||_F^2 (= tr X^2, X symmetric) into tr[0], tr[1] (zeroed before).
@@ -133,14 +137,22 @@ __global__ void k_sp2_start(const double* __restrict__ f, const double* __restri
     const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     double d = 0.0, q = 0.0;
     if (t < (size_t)n * n) {
-        const double lo = bounds[0], hi = bounds[1];
+        const double hi = bounds[1];
         const int i = (int)(t % n), j = (int)(t / n);
-        const double v = ((i == j ? hi : 0.0) - f[t]) / (hi - lo);
+        const double v = ((i == j ? hi : 0.0) - f[t]) / sp2_range(bounds[0], hi);
         x[t] = v;
         d = i == j ? v : 0.0;
         q = v * v;
     }
     block_add2(d, q, tr);
+}
+
+// Whether the purification has to be replaced by an eigensolve: X is not
+// idempotent after the last step (no gap at the occupation: an open shell
+// asked for as a closed one), or is a projector of another rank (an eigenvalue
+// that maps to exactly 0 or 1 stays there).  NaN in F stays NaN.
+__host__ __device__ __forceinline__ bool sp2_failed(bool idempotent, double tr, double nocc) {
+    return tr == tr && !(idempotent && fabs(tr - nocc) < 0.5);
 }
 
 // One SP2 step: X <- X^2 when that brings the trace nearer nocc, else
@@ -207,9 +219,11 @@ __device__ __forceinline__ double cta_reduce(double v, double* red) {
     return v;
 }
 
-// x0, x1: n x n buffers; the projector ends up in x0.  *steps += steps done.
+// x0, x1: n x n buffers; the projector ends up in x0.  *steps += steps done;
+// *failed: 1 if x0 is not a projector of rank nocc (sp2_failed), else 0.
 __global__ void __cluster_dims__(SP2C, 1, 1) __launch_bounds__(SP2T)
-    k_sp2_cluster(const double* __restrict__ f, int n, double nocc, double tol, double* x0, double* x1, int* steps) {
+    k_sp2_cluster(const double* __restrict__ f, int n, double nocc, double tol, double* x0, double* x1, int* steps,
+                  int* failed) {
     extern __shared__ __align__(16) double X[];
     __shared__ double red[SP2T / 32];
     const int ld = sp2_ld(n), nt = (n + 7) / 8, np = nt * 8;
@@ -236,7 +250,7 @@ __global__ void __cluster_dims__(SP2C, 1, 1) __launch_bounds__(SP2T)
     double tr = 0.0, sq = 0.0;
     for (int t = tid; t < n * n; t += SP2T) {
         const int i = t % n, j = t / n;
-        const double v = ((i == j ? hi : 0.0) - X[j * ld + i]) / (hi - lo);
+        const double v = ((i == j ? hi : 0.0) - X[j * ld + i]) / sp2_range(lo, hi);
         X[j * ld + i] = v;
         tr += i == j ? v : 0.0;
         sq += v * v;
@@ -289,9 +303,12 @@ __global__ void __cluster_dims__(SP2C, 1, 1) __launch_bounds__(SP2T)
         ++step;
     }
     // an odd number of steps left the result in x1; x0 is no longer read
-    if (step & 1 || step == 0)
+    if (step & 1)
         for (int t = rank * SP2T + tid; t < n * n; t += SP2C * SP2T) x0[t] = X[(t / n) * ld + t % n];
-    if (rank == 0 && tid == 0) *steps += step;
+    if (rank == 0 && tid == 0) {
+        *steps += step;
+        *failed = sp2_failed(more >= 0, tr, nocc);
+    }
 }
 
 // The cycle's scalars in one pass: sum P H, sum P F, <R_new, R_j> for the
@@ -359,6 +376,7 @@ struct hfgpu_scf {
     int lwork = 0;
     int* info = nullptr;
     int* nsteps = nullptr;      // purification steps of the one-launch form, all cycles
+    int* sp2_bad = nullptr;     // page-locked, read by the host: the last purification failed
     void* blas_ws = nullptr;
     void* arena = nullptr;       // one stream-ordered allocation holding every buffer above
     CycleScalars* sc = nullptr;  // device
@@ -450,9 +468,15 @@ int density_from_cob(hfgpu_scf* s, double* P) {
 // D is the projector on the nocc lowest eigenvectors of Fo, the density the
 // eigenvectors give (direct_hartreefock.f90:204-218), reached with matrix
 // products only.  Each step's choice is made on the device; the host checks
-// idempotency every few steps.
+// idempotency every few steps.  Once the stream has been waited for,
+// *s->sp2_bad says whether P is something else than that density.
 int density_by_purification(hfgpu_scf* s, const double* Fo, double* P) {
     const int nb = s->nb;
+    *s->sp2_bad = 0;  // nothing that writes it is in flight
+    // every orbital occupied (He and Ne in a minimal basis): D = 1.  The
+    // highest occupied eigenvalue may lie on the upper bound, where it maps
+    // to 0, and for nb = 1 the bounds coincide
+    if (s->nocc == nb) return gemm(s, false, true, 2.0, s->X, s->X, 0.0, P);
     const size_t n2 = (size_t)nb * nb;
     const unsigned blocks = (unsigned)((n2 + 255) / 256);
     double* X = s->T1;
@@ -462,7 +486,7 @@ int density_by_purification(hfgpu_scf* s, const double* Fo, double* P) {
     double* lo = s->aux + 8;
     if (nb <= SP2_MAXN) {  // one launch; larger matrices fill the GPU with a product per step
         k_sp2_cluster<<<SP2C, SP2T, (size_t)((nb + 7) / 8 * 8) * sp2_ld(nb) * sizeof(double), s->st>>>(
-            Fo, nb, (double)s->nocc, 1e-11 * std::max(1, s->nocc), X, X2, s->nsteps);
+            Fo, nb, (double)s->nocc, 1e-11 * std::max(1, s->nocc), X, X2, s->nsteps, s->sp2_bad);
         SCF_CUDA(cudaGetLastError());
         SCF_RC(gemm(s, false, false, 1.0, s->X, X, 0.0, X2));
         return gemm(s, false, true, 2.0, X2, s->X, 0.0, P);
@@ -475,8 +499,10 @@ int density_by_purification(hfgpu_scf* s, const double* Fo, double* P) {
     // the first check after 16 steps (the start needs ~log2 of the spectral
     // range over the gap of them), then every 4; each step is the product X^2
     // and one update kernel that also forms the next step's traces
-    constexpr int FIRST = 16, BLOCK = 4, MAXSTEP = 160;
-    for (int step = 0; step < MAXSTEP;) {
+    constexpr int FIRST = 16, BLOCK = 4;
+    bool idempotent = false;
+    double h_tr[2] = {0.0, 0.0};
+    for (int step = 0; step < SP2_MAXSTEP && !idempotent;) {
         const int nstep = step == 0 ? FIRST : BLOCK;
         for (int k = 0; k < nstep; ++k) {
             const int q = step + k;
@@ -487,12 +513,12 @@ int density_by_purification(hfgpu_scf* s, const double* Fo, double* P) {
         step += nstep;
         s->sp2_steps += nstep;
         SCF_CUDA(cudaGetLastError());
-        double h_tr[2];
         SCF_CUDA(cudaMemcpyAsync(h_tr, tr + 2 * (step % 3), sizeof(h_tr), cudaMemcpyDeviceToHost, s->st));
         SCF_CUDA(cudaStreamSynchronize(s->st));
         // tr X - tr X^2 = sum x_k (1 - x_k) over the eigenvalues: zero for a projector
-        if (std::fabs(h_tr[0] - h_tr[1]) < 1e-11 * std::max(1, s->nocc)) break;
+        idempotent = std::fabs(h_tr[0] - h_tr[1]) < 1e-11 * std::max(1, s->nocc);
     }
+    *s->sp2_bad = sp2_failed(idempotent, h_tr[0], (double)s->nocc);
     // P = 2 X_s D X_s^T with X_s = S^-1/2
     SCF_RC(gemm(s, false, false, 1.0, s->X, X, 0.0, X2));
     SCF_RC(gemm(s, false, true, 2.0, X2, s->X, 0.0, P));
@@ -527,10 +553,13 @@ bool small_solve(std::vector<double>& A, std::vector<double>& b, int n) {
 
 // cuBLAS / cuSOLVER handles are pooled across jobs: creating them costs
 // milliseconds and may allocate, so a served job borrows a pair and gives it
-// back when it ends.
+// back when it ends.  With them goes the page-locked word by which the
+// purification kernel tells the host that it failed (a copy of it back each
+// cycle cost 12 us).
 struct LinAlg {
     cublasHandle_t blas;
     cusolverDnHandle_t sol;
+    int* flag;
 };
 std::mutex g_pool_mu;
 std::vector<LinAlg> g_pool;
@@ -541,6 +570,7 @@ int acquire_linalg(hfgpu_scf* s) {
         if (!g_pool.empty()) {
             s->blas = g_pool.back().blas;
             s->sol = g_pool.back().sol;
+            s->sp2_bad = g_pool.back().flag;
             g_pool.pop_back();
         }
     }
@@ -548,6 +578,7 @@ int acquire_linalg(hfgpu_scf* s) {
         std::lock_guard<std::recursive_mutex> lk(hfgpu::device_mutex());  // creation may allocate
         SCF_BLAS(cublasCreate(&s->blas));
         SCF_SOLVER(cusolverDnCreate(&s->sol));
+        SCF_CUDA(cudaHostAlloc((void**)&s->sp2_bad, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
     }
     SCF_BLAS(cublasSetStream(s->blas, s->st));
     SCF_BLAS(cublasSetPointerMode(s->blas, CUBLAS_POINTER_MODE_HOST));
@@ -561,12 +592,13 @@ void release(hfgpu_scf* s) {
         if (e) cudaEventDestroy(e);
     if (s->arena) cudaFreeAsync(s->arena, s->st);
     if (s->st) cudaStreamSynchronize(s->st);
-    if (s->blas && s->sol) {
+    if (s->blas && s->sol && s->sp2_bad) {
         std::lock_guard<std::mutex> lk(g_pool_mu);
-        g_pool.push_back({s->blas, s->sol});
+        g_pool.push_back({s->blas, s->sol, s->sp2_bad});
     } else {
         if (s->blas) cublasDestroy(s->blas);
         if (s->sol) cusolverDnDestroy(s->sol);
+        if (s->sp2_bad) cudaFreeHost(s->sp2_bad);
     }
     delete s;
 }
@@ -821,6 +853,13 @@ int run(hfgpu_scf* s, const hfgpu_scf_params& prm, hfgpu_scf_result* res) {
         else SCF_RC(density_by_purification(s, s->Fob, s->P));
         SCF_CUDA(cudaEventRecord(s->ev[3], s->st));
         SCF_CUDA(cudaEventSynchronize(s->ev[3]));
+        if (!vectors && *(volatile int*)s->sp2_bad) {
+            SCF_RC(eigensolve(s, s->Fob));
+            SCF_RC(density_from_cob(s, s->P));
+            s->eigs_current = true;
+            SCF_CUDA(cudaEventRecord(s->ev[3], s->st));
+            SCF_CUDA(cudaEventSynchronize(s->ev[3]));
+        }
         float mb = 0.f, md = 0.f;
         cudaEventElapsedTime(&mb, s->ev[0], s->ev[1]);
         cudaEventElapsedTime(&md, s->ev[2], s->ev[3]);

@@ -20,11 +20,13 @@ the occupied projector is formed by second-order spectral projection
 Gershgorin-scaled Fock matrix, each step replaces X by X^2 or 2X - X^2,
 whichever keeps trace(X) nearer the number of occupied orbitals.  For a
 closed-shell system with a HOMO-LUMO gap this converges quadratically to the
-same projector the eigenvectors give, using FP64 matrix products only.
+same projector the eigenvectors give, using FP64 matrix products only.  Where
+it does not (no gap), the cycle's density comes from the eigenvectors, outside
+the graph.
 
 The protocol's decisions (DIIS start, threshold drop, full vs incremental
 build, convergence) are made on the device where they depend on this cycle's
-numbers; the host reads five scalars per cycle and picks the next graph:
+numbers; the host reads six scalars per cycle and picks the next graph:
 (full | incremental) x (loose | tight threshold), plus the first cycle, whose
 Fock build (the Schwarz pass) runs through the host interface.
 """
@@ -74,7 +76,8 @@ class DeviceSCF:
         self.rhs0 = z(NDIIS + 1)
         self.rhs0[NDIIS] = -1.0  # the Lagrange row of the DIIS system
         self.status = torch.zeros(1, dtype=torch.int32, device=self.dev)
-        self.out = z(5)  # eelec, resmax, deltap, threshold-drop flag, nusediis
+        self.out = z(6)  # eelec, resmax, deltap, threshold-drop flag, nusediis, purification failed
+        self.fob = z(nb, nb)  # the (extrapolated) orthogonal Fock matrix of the last cycle
         self.idx = torch.arange(NDIIS, device=self.dev)
         self._graphs: Dict[tuple, object] = {}
         self.enuc = mol.nuclear_repulsion()
@@ -139,7 +142,8 @@ class DeviceSCF:
         fob = torch.where(use & ok, torch.einsum("j,jab->ab", c, self.FO), fob)
         self.n.copy_(torch.where(use & ~ok, torch.zeros_like(n), n))
         # density: occupied projector of fob by SP2, back to the AO basis
-        D = self._sp2(fob)
+        D, failed = self._sp2(fob)
+        self.fob.copy_(fob)
         Pn = 2.0 * (X @ D @ X)
         self.Pnew.copy_(0.5 * (Pn + Pn.T))
         deltap = (P - self.Pold).abs().max()
@@ -149,21 +153,37 @@ class DeviceSCF:
         self.out[2] = deltap
         self.out[3] = drop.to(torch.float64)
         self.out[4] = self.n.to(torch.float64)
+        self.out[5] = failed
 
     def _sp2(self, F):
+        """(projector on the nocc lowest eigenvectors of F, 1.0 if it is not
+        one).  It fails without a gap at the occupation (a degenerate open
+        shell), or when an eigenvalue on a bound of the spectrum maps to
+        exactly 0 or 1 on the wrong side."""
         torch = self.torch
         nb = self.nb
         eye = torch.eye(nb, dtype=torch.float64, device=self.dev)
+        nocc = float(self.nocc)
+        if self.nocc == nb:  # every orbital occupied
+            return eye, torch.zeros((), dtype=torch.float64, device=self.dev)
         off = F.abs().sum(dim=1) - F.diagonal().abs()
         emin = (F.diagonal() - off).min()
         emax = (F.diagonal() + off).max()
-        Xk = (emax * eye - F) / (emax - emin)
-        nocc = float(self.nocc)
+        width = torch.where(emax > emin, emax - emin, torch.ones_like(emax))
+        Xk = (emax * eye - F) / width
         for _ in range(self.sp2_steps):
             X2 = Xk @ Xk
             tr, tr2 = Xk.diagonal().sum(), X2.diagonal().sum()
             Xk = torch.where(torch.abs(tr2 - nocc) < torch.abs(2.0 * tr - tr2 - nocc), X2, 2.0 * Xk - X2)
-        return Xk
+        tr, tr2 = Xk.diagonal().sum(), (Xk * Xk).sum()
+        good = (torch.abs(tr - tr2) < 1e-9 * nocc) & (torch.abs(tr - nocc) < 0.5)
+        return Xk, ((tr == tr) & ~good).to(torch.float64)  # NaN in F stays NaN
+
+    def _density_from_eigenvectors(self):
+        """The density where the purification failed (direct_hartreefock.f90:204-218)."""
+        _, U = self.torch.linalg.eigh(self.fob)
+        C = self.X @ U[:, :self.nocc]
+        self.Pnew.copy_(2.0 * (C @ C.T))
 
     def _cycle(self, kind: str, thr: float, fdifffac: float, cut: float, loose: bool):
         torch = self.torch
@@ -230,7 +250,7 @@ class DeviceSCF:
                     if nfull == 15:
                         fullfock = True
                 self._cycle(kind, thresh, fdifffac, fp32_cutoff if kind == "delta" else 0.0, loose)
-            eelec, resmax, deltap, drop, _ = (float(x) for x in self.out.cpu())
+            eelec, resmax, deltap, drop, _, failed = (float(x) for x in self.out.cpu())
             deltae = eelec - eeold
             if drop > 0.5:  # direct_hartreefock.f90:152-160
                 fullfock = True
@@ -242,6 +262,8 @@ class DeviceSCF:
             if abs(deltae) < conve and deltap < conv and it > 1:
                 converged = True
                 break
+            if failed:
+                self._density_from_eigenvectors()
             self.Pold.copy_(self.P)
             self.P.copy_(self.Pnew)
         return SCFResult(energy=eelec + self.enuc, eelec=eelec, enuc=self.enuc, converged=converged,
