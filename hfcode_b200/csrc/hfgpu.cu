@@ -1354,6 +1354,12 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
         h->warp_scatter = 16LL * h->nsm;
         h->direct_blocks = 64LL * h->nsm;
         if (const char* e = getenv("HFGPU_DIRECT")) h->direct_blocks = atoll(e);
+        // one form for every list: "single", one thread per quartet, or
+        // "grouped", the lanes of a warp together
+        if (const char* e = getenv("HFGPU_SCATTER")) {
+            if (strcmp(e, "single") == 0) h->warp_scatter = 0;
+            if (strcmp(e, "grouped") == 0) h->warp_scatter = INT64_MAX;
+        }
         if (const char* e = getenv("HFGPU_WARP_SCATTER")) h->warp_scatter = atoll(e);
         if (const char* e = getenv("HFGPU_STREAMS")) h->nstreams = std::max(1, std::min(NSTREAM, atoi(e)));
     }
