@@ -1035,9 +1035,13 @@ unsigned walk_blocks(long long need, long long fill, bool capture) {
     return (unsigned)std::max<long long>(1, capture ? std::min(need, fill) : need);
 }
 
-// Blocks of a direct class's list of (at most) n quartets.
+// Blocks of a direct class's list of n quartets; in a capture an upper bound,
+// from the candidates.  direct_grid is what is launched.
 long long direct_need(const hfgpu_handle* h, int c, int prec, long long n, bool capture) {
-    return walk_blocks(((capture ? n : h->nunit[2 * c + prec]) + WPB - 1) / WPB, 8LL * h->nsm, capture);
+    return ((capture ? n : h->nunit[2 * c + prec]) + WPB - 1) / WPB;
+}
+unsigned direct_grid(const hfgpu_handle* h, int c, int prec, long long n, bool capture) {
+    return walk_blocks(direct_need(h, c, prec, n, capture), 8LL * h->nsm, capture);
 }
 
 // Staged class: chunks of the quartet list through the accumulator roles
@@ -1203,7 +1207,11 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
         for (int k = 0; k < h->nstreams; ++k) HF_CHECK(cudaStreamWaitEvent(h->aux[k], h->fork, 0));
     }
     double load[NSTREAM] = {};
-    // the direct classes of a small build side by side in one launch per precision
+    // The direct classes of a small build side by side in one launch per
+    // precision.  Small by the work, not by the grid: a capture's grids are
+    // capped, and by those every build with few direct classes would be small
+    // (C60 in STO-3G with split sp shells: 16.4 ms recorded in one launch,
+    // 14.5-15.2 with a launch per class; n-C20H42 in STO-3G 0.52 and 0.48).
     long long direct_blocks = 0;
     for (const Item& it : items)
         if (CLASS_KERNELS[it.c].mode == 0) direct_blocks += direct_need(h, it.c, it.prec, it.n, capture);
@@ -1221,7 +1229,7 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
             d.ket = h->d_apairs[K.ki];
             d.stats = h->d_stats + it.c;
             d.block0 = blocks;
-            d.blocks = (int)direct_need(h, it.c, prec, it.n, capture);
+            d.blocks = (int)direct_grid(h, it.c, prec, it.n, capture);
             blocks += d.blocks;
             w += it.w;
         }
@@ -1269,7 +1277,7 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
             a.thr = thr;
             a.jonly = jonly;
             a.stats = h->d_stats + c;
-            const unsigned blocks = (unsigned)direct_need(h, c, prec, n, capture);
+            const unsigned blocks = direct_grid(h, c, prec, n, capture);
             ++h->launches;
             (prec ? K.nd32 : K.nd64)<<<blocks, ND_THREADS, 0, st>>>(a);
             HF_CHECK(cudaGetLastError());
