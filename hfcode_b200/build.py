@@ -10,6 +10,7 @@ from __future__ import annotations
 import concurrent.futures as cf
 import glob
 import os
+import re
 import subprocess
 import sys
 
@@ -28,6 +29,14 @@ def _newer(target: str, deps) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _includes(src: str):
+    """The generated headers a source includes from its own folder."""
+    here = os.path.dirname(src)
+    with open(src) as fh:
+        names = re.findall(r'^#include "([^"/]+)"', fh.read(), re.M)
+    return [os.path.join(here, n) for n in names if os.path.exists(os.path.join(here, n))]
 
 
 def _compile(src: str, obj: str, deps) -> str:
@@ -63,8 +72,7 @@ def build(jobs: int = 0, verbose: bool = True) -> str:
     objs = [os.path.join(BUILD, os.path.splitext(os.path.basename(s))[0] + ".o") for s in srcs]
     jobs = jobs or max(1, min(len(srcs), os.cpu_count() or 4))
     with cf.ThreadPoolExecutor(jobs) as ex:
-        futs = [ex.submit(_compile, s, o, common + ([s[:-3] + ".cuh"] if os.path.exists(s[:-3] + ".cuh") else []))
-                for s, o in zip(srcs, objs)]
+        futs = [ex.submit(_compile, s, o, common + _includes(s)) for s, o in zip(srcs, objs)]
         for f in futs:
             done = f.result()
             if done and verbose:
