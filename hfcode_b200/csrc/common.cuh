@@ -199,7 +199,7 @@ struct NDArgs {
     const GPair* bra;
     const GPair* ket;
     PrimSoA prims;
-    const double* boys;     // global table, [M][225][8]
+    const double* boys;     // Boys tables of every order, BOYS_BLK values each (types.cuh)
     const float* boysf;
     const double* Pb;       // density in shell-pair blocks
     double* G;              // in shell-pair blocks
@@ -475,10 +475,6 @@ __device__ __forceinline__ uint2 staged_quartet(const StagedArgs& a, int t) {
 // barrier is needed; cp.async.wait_group bounds each wait by the thread's own
 // copies.  P_bc and P_bd, needed for every i, are staged once in shared
 // memory as well.
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
@@ -651,9 +647,9 @@ __global__ void __launch_bounds__(ND_THREADS, sizeof(E) == 4 ? 3 : 2) k_scatter_
     const int cnt = staged_count(a);
     const int w0 = t - (threadIdx.x & 31);  // first quartet of this warp
     if (w0 >= cnt) return;                  // a warp with no quartet (whole warps only)
-    // every lane of the warp runs the scatter so that the J_ab sums can be
-    // reduced across the warp; a lane past the end works on the warp's first
-    // quartet and writes nothing
+    // every lane of the warp runs the scatter, because the lanes add the
+    // warp's block elements together (walk_add); a lane past the end works on
+    // the warp's first quartet and adds nothing
     const bool valid = t < cnt;
     const int tq = valid ? t : w0;
     double m = 0.0;

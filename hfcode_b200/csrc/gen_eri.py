@@ -22,7 +22,7 @@ horizontal recurrence always moves angular momentum from A to B and from C to
 D.  The output block is out[((i*nB + j)*nC + k)*nD + l] in this order, each
 shell's functions in the reference's component order (L: s,x,y,z).
 
-Run as a script to regenerate ``generated/eri_classes.cuh``.
+Run as a script to regenerate ``generated/``.
 """
 from __future__ import annotations
 
@@ -328,14 +328,9 @@ class ClassGen:
             s |= self.leaves(c4)
         return s
 
-    def partition(self, acc_max: int, out_max: int, b_split=None):
+    def partition(self, acc_max: int, out_max: int):
         """Greedy split of the outputs (flat order) into roles whose
-        accumulator and output counts fit the register budget; or, with
-        `b_split`, one role per function of the first shell and block of the
-        second's."""
-        if b_split:
-            return [[n for n, o in enumerate(self.outputs) if o[0] == i and o[1] in blk]
-                    for i in range(self.nf[0]) for blk in b_split]
+        accumulator and output counts fit the register budget."""
         groups, cur, cur_acc = [], [], set()
         for n, o in enumerate(self.outputs):
             lv = self.out_leaves(o)
@@ -599,49 +594,6 @@ class ClassGen:
         self.flops_quartet = 2 * st["hrr"] + 2 * st["sph"] + 12 * self.nout
         self.nvrr, self.nhrr = st["vrr"], st["hrr"]
 
-    # ------------------------------------------------------------- scatter
-    def emit_scatter(self, fname: str, outs: List[int]) -> str:
-        """J/K scatter of the outputs `outs` with uniform weight s into the
-        one-triangle buffer G (F += G + G^T later); P is column-major."""
-        o4 = [self.outputs[n] for n in outs]
-        lines = [f"template <typename E>",
-                 f"__device__ __forceinline__ void {fname}(const E* __restrict__ e, double s, const GPair& bra, "
-                 f"const GPair& ket, const double* __restrict__ P, double* __restrict__ G, int nb, bool jonly)",
-                 "{",
-                 "    const int a0 = bra.aoa, b0 = bra.aob, c0 = ket.aoa, d0 = ket.aob;",
-                 "    const double s2 = 2.0 * s, hs = -0.5 * s;"]
-        loaded = set()
-        org = {"a": "a0", "b": "b0", "c": "c0", "d": "d0"}
-
-        def pv(x, i, y, j):
-            nm = f"p{x}{i}{y}{j}"
-            if nm not in loaded:
-                loaded.add(nm)
-                lines.append(f"    const double {nm} = __ldg(P + ({org[x]} + {i}) + (size_t)({org[y]} + {j}) * nb);")
-            return nm
-
-        def block(rowx, rowi, colx, coli, px, pi, qx, qi, scale, tgt):
-            groups: Dict[Tuple[int, int], List[Tuple[int, int]]] = {}
-            for r, o in enumerate(o4):
-                key = (o[rowi], o[coli])
-                groups.setdefault(key, []).append((r, o))
-            for (i, j), lst in groups.items():
-                terms = [f"{pv(px, o[pi], qx, o[qi])} * (double)e[{r}]" for r, o in lst]
-                lines.append(f"    atomicAdd(G + ({org[rowx]} + {i}) + (size_t)({org[colx]} + {j}) * nb, "
-                             f"{scale} * ({' + '.join(terms)}));")
-
-        # J_ab <- P_cd, J_cd <- P_ab
-        block("a", 0, "b", 1, "c", 2, "d", 3, "s2", "J")
-        block("c", 2, "d", 3, "a", 0, "b", 1, "s2", "J")
-        lines.append("    if (jonly) return;")
-        # K_ac <- P_bd, K_ad <- P_bc, K_bc <- P_ad, K_bd <- P_ac
-        block("a", 0, "c", 2, "b", 1, "d", 3, "hs", "K")
-        block("a", 0, "d", 3, "b", 1, "c", 2, "hs", "K")
-        block("b", 1, "c", 2, "a", 0, "d", 3, "hs", "K")
-        block("b", 1, "d", 3, "a", 0, "c", 2, "hs", "K")
-        lines.append("}")
-        return "\n".join(lines)
-
 
 ACC_MAX = 64        # accumulators per output role (register budget)
 OUT_MAX = 32        # outputs per output role
@@ -649,6 +601,7 @@ MAX_ROLES2 = 12     # beyond this, the class goes through the accumulator stage
 ACC_GROUP = 48      # accumulators per stage-A role (d-heavy classes)
 OUT_GROUP3 = 25     # outputs per stage-B role (d-heavy classes)
 MAXR = 64           # role slots in ClassKernels
+MAXDIRECT = 64      # list slots in NDAllArgs
 
 # Per-class shape overrides (measured on the device; see tuning.json beside
 # this file): {"<tag>": {"acc_max": .., "out_max": .., "max_roles2": ..,
@@ -739,7 +692,9 @@ def class_source(ci: int, bi: int, ki: int):
     quartet class; returns (cuh_text, cu_text, info).
 
     Three shapes:
-      direct  one thread per quartet computes the whole block (k_nondiag);
+      direct  one warp per work unit: each lane computes the whole block of a
+              quartet, or its share of the primitive loops where the unit
+              spreads a quartet over several lanes (k_nondiag);
       staged2 the outputs are split into roles, one kernel launch per role
               (uniform code per launch), each writing its outputs and their
               max to a scratch buffer; k_scatter_staged applies the
@@ -752,7 +707,7 @@ def class_source(ci: int, bi: int, ki: int):
     g32 = ClassGen(PAIR_TYPES[bi], PAIR_TYPES[ki], "float", suffix="_f32")
     g.flop_model()
     prm = class_params(g.tag)
-    roles = g.partition(prm["acc_max"], prm["out_max"], prm.get("b_split"))
+    roles = g.partition(prm["acc_max"], prm["out_max"])
     funcs, kern = [], []
     reg = []
     NA, NB, NC, ND = g.nf
@@ -1018,7 +973,7 @@ def direct_all(outdir: str, infos: dict):
         path = os.path.join(outdir, f"direct_all{'32' if f32 else '64'}.cu")
         write_if_changed(path, "\n".join(lines))
         out.append(path)
-    assert len(direct) <= 64
+    assert len(direct) <= MAXDIRECT
     return out
 
 
@@ -1031,9 +986,7 @@ def main(outdir: str):
         flops[ci] = info
         base = os.path.join(outdir, f"cls_{ci:02d}_{info['tag']}")
         for ext, text in ((".cuh", cuh), (".cu", cu)):
-            if not os.path.exists(base + ext) or open(base + ext).read() != text:
-                with open(base + ext, "w") as fh:
-                    fh.write(text)
+            write_if_changed(base + ext, text)
         names.append(base + ".cu")
     names += direct_all(outdir, flops)
     # host dispatch used by the host-compiled check of the generated code
@@ -1104,23 +1057,15 @@ def main(outdir: str):
            "#define HF_FOR_EACH_CLASS(X) " + " ".join(f"X({c})" for c in range(len(cl))),
            "#define HF_PAIR_NAMES " + ", ".join(f'"{a}{b}"' for a, b in PAIR_TYPES), ""]
     ct = os.path.join(outdir, "class_table.inc")
-    if not os.path.exists(ct) or open(ct).read() != "\n".join(tab):
-        with open(ct, "w") as fh:
-            fh.write("\n".join(tab))
+    write_if_changed(ct, "\n".join(tab))
     ai = os.path.join(outdir, "all_classes.inc")
-    if not os.path.exists(ai) or open(ai).read() != inc:
-        with open(ai, "w") as fh:
-            fh.write(inc)
+    write_if_changed(ai, inc)
     hd = os.path.join(outdir, "host_dispatch.inc")
-    if not os.path.exists(hd) or open(hd).read() != txt:
-        with open(hd, "w") as fh:
-            fh.write(txt)
+    write_if_changed(hd, txt)
     import json
     fl = os.path.join(outdir, "class_flops.json")
     txt = json.dumps(flops, indent=1)
-    if not os.path.exists(fl) or open(fl).read() != txt:
-        with open(fl, "w") as fh:
-            fh.write(txt)
+    write_if_changed(fl, txt)
     return names
 
 

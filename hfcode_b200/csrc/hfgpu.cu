@@ -118,7 +118,7 @@ namespace {
 
 constexpr double SHTHRESH = 1e-11;      // molprops.f90:163
 constexpr int NSTREAM = 8;              // class streams a handle creates (HFGPU_STREAMS of them used, default 4)
-// bra and ket pair types of the 21 quartet classes (pair types i <= j, row by row)
+// bra and ket pair types of the quartet classes, in the generator's class order
 __constant__ int CLS_BI[NCLS] = {HF_CLASS_BI_LIST};
 __constant__ int CLS_KI[NCLS] = {HF_CLASS_KI_LIST};
 
@@ -441,11 +441,6 @@ __global__ void k_symm(double* __restrict__ F, const double* __restrict__ G, con
 }
 
 // ------------------------------------------------------------- host ----
-struct DevBuf {
-    void* p = nullptr;
-    size_t n = 0;
-};
-
 }  // namespace
 
 struct hfgpu_handle {
@@ -667,7 +662,7 @@ int launch_symm(hfgpu_handle* h, double* F, const double* G = nullptr) {
 // runs the same role's code (these FP64 recursions are long straight-line
 // programs, and an SM running several of them thrashes its instruction
 // cache); small chunks gain more from filling the SMs and launching less.
-bool merge_roles(const hfgpu_handle* h, const ClassKernels& K, int blocks, int roles) {
+bool merge_roles(const hfgpu_handle* h, int blocks, int roles) {
     return (long long)blocks * roles <= h->merge_blocks;
 }
 
@@ -831,8 +826,8 @@ int build_active(hfgpu_handle* h) {
             int nx = h->pairs[t][x].g.np, ny = h->pairs[t][y].g.np;
             if (nx != ny) return nx > ny;
             // within a primitive-count group by first shell, so the 32
-            // quartets of a warp mostly share it (the staged scatter then
-            // adds their K blocks with one atomic per element)
+            // quartets of a warp mostly share it (the scatter adds the runs
+            // of quartets that share a block with one atomic per element)
             const int sx = h->pairs[t][x].g.sa, sy = h->pairs[t][y].g.sa;
             if (sx != sy) return sx < sy;
             return h->schw[t][x] > h->schw[t][y];
@@ -1081,7 +1076,7 @@ int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, d
         a.stats = h->d_stats + c;
         const int blocks = (m + ND_THREADS - 1) / ND_THREADS;
         const int na = prec ? K.nrole_a32 : K.nrole_a;
-        if (merge_roles(h, K, blocks, std::max(na, a.nroles))) {
+        if (merge_roles(h, blocks, std::max(na, a.nroles))) {
             // a small list: every role of a stage in one launch, side by side,
             // the primitive-loop stage on the class's work units
             a.list = unit_list(h, c, prec);
@@ -1126,8 +1121,8 @@ int run_staged(hfgpu_handle* h, int c, int prec, long long n, const double* P, d
     return HFGPU_OK;
 }
 
-// Off-diagonal build: the two screening passes with device-side offsets,
-// then the class kernels on the handle's concurrent class streams.  With capture set,
+// Off-diagonal build: the screen, the list offsets and the expansion into
+// lists, then the class kernels on the handle's concurrent class streams.  With capture set,
 // nothing is read back on the host: every launch is sized by the class's
 // candidate count (an upper bound) and the kernels read the surviving count
 // from d_ncls, so the whole sequence can be recorded into a CUDA graph.
@@ -1170,7 +1165,7 @@ int run_non_diag(hfgpu_handle* h, const double* P, double thr, int jonly, double
         k_expand<<<blocks, 256, 0, h->stream>>>(sa);  // compacted write
         HF_CHECK(cudaGetLastError());
     }
-    {  // the density in shell-pair blocks for the staged scatter
+    {  // the density in shell-pair blocks for the scatters
         const long long n = (long long)h->nb * h->nb;
         ++h->launches;
         k_pblock<<<(int)((n + 255) / 256), 256, 0, h->stream>>>(P, h->d_Pb, h->d_aomap, h->d_nfsh, h->d_boff, h->nb,
@@ -1359,7 +1354,16 @@ int hfgpu_init(const hfgpu_basis* B, hfgpu_handle** out) {
         // 10.8 jobs/s without merging, 14.9 at 2 x SMs, 23.9 at 8 x SMs
         h->merge_blocks = 8LL * h->nsm;
         if (const char* e = getenv("HFGPU_MERGE_BLOCKS")) h->merge_blocks = atoll(e);
+        // 16 quartets per SM.  At 0 / 4 / 8 / 16 / 32 / 64 / 128 per SM:
+        // benzene recorded 499, 499, 482, 468, 475, 505, 536 us, mixed 703,
+        // 631, 651, 613, 624, 648 us; C8H18 916, 878, 890, 887, 876, 921, 972
+        // us; (H2O)12 882, 856, 862, 877, 891, 905, 957 us.  From C16H34 on the
+        // choice is within 1% up to 64
         h->warp_scatter = 16LL * h->nsm;
+        // 64 blocks per SM.  A launch per class against one launch: water in
+        // STO-3G 106 and 87 us, benzene 567 and 530; C16H34 3.06 and 3.22 ms,
+        // C60 in STO-3G with split sp shells 14.3 and 15.9 ms.  In between flat
+        // but for n-C20H42 in STO-3G, 524 us up to 32 and 557 from 64 on
         h->direct_blocks = 64LL * h->nsm;
         if (const char* e = getenv("HFGPU_DIRECT")) h->direct_blocks = atoll(e);
         // one form for every list: "single", one thread per quartet, or
