@@ -13,8 +13,9 @@
  * orthogonalised Fock matrix; here that projector is formed by second-order
  * spectral projection (SP2, matrix products only), and cuSOLVER's syevd
  * (dsyev's role) runs only where eigenvectors are needed: the
- * core-Hamiltonian guess, cycles with the level shift on, and the orbital
- * energies on request.  A few scalars per cycle come back to the host, where
+ * core-Hamiltonian guess, cycles with the level shift on, cycles whose matrix
+ * has no gap at the occupation, and the orbital energies on request.  A few
+ * scalars per cycle come back to the host, where
  * the protocol's decisions are taken as the reference takes them.
  *
  * One job per builder handle (the job uses the handle's stream); jobs on
