@@ -188,8 +188,8 @@ struct ClassStats {
 
 // Unit u of the list: false past the end (see unit_place).
 __device__ __forceinline__ bool unit_of(const UnitList& L, int u, Unit& w) {
-    const long long at = unit_place(L, u, threadIdx.x & 31, w);
-    if (at < 0) return false;
+    long long at;
+    if (!unit_place(L, u, threadIdx.x & 31, w, at)) return false;
     w.q = L.quartets[at];
     return true;
 }
@@ -436,9 +436,15 @@ __device__ __forceinline__ void chunk_units(const StagedArgs& a, int& u0, int& u
 // Unit u of a one-launch stage (chunk_units).
 __device__ __forceinline__ void stage_unit(const StagedArgs& a, int u, Unit& w) {
     if (a.list.subs) {
-        unit_of(a.list, u, w);
-        w.t -= a.q0;  // entries of other chunks are not stored
-        w.store = w.store && w.t >= 0 && w.t < a.n;
+        // the entry is counted in 64 bits, but held in 32: the extra register
+        // cost the primitive-loop stages 12 bytes of spills, 1-2% of a small
+        // build
+        long long at = 0;
+        unit_place(a.list, u, threadIdx.x & 31, w, at);
+        const long long t = at - list_start(a.list) - a.q0;
+        w.q = a.list.quartets[at];
+        w.store = w.store && t >= 0 && t < a.n;  // entries of other chunks are not stored
+        w.t = (int)t;
         return;
     }
     // diagonal builders: two pairs per warp, their at most 9 x 9 primitive

@@ -33,7 +33,7 @@ struct ScreenSub {
 // chain the time of the whole kernel for a small molecule (benzene SS|SS:
 // 255 us at 66 blocks).
 struct Unit {
-    long long t;       // entry within the class's list of this precision (stage_unit: within the chunk)
+    int t;             // entry within the chunk (stage_unit)
     bool store;        // this lane writes the quartet's results
     uint2 q;           // (bra, ket)
     LaneSplit ls;
@@ -55,13 +55,13 @@ __device__ __forceinline__ long long list_start(const UnitList& L) {
     return L.coff + (L.prec ? (long long)L.ncls[2 * L.cls] : 0);
 }
 
-// Lane `lane` of unit u of the list: everything but the quartet itself, whose
-// place in the quartet buffer is returned; -1 past the end.  The lanes
-// without a quartet (the tail of a sub-class) repeat the sub-class's last one
-// and do not store.
-__device__ __forceinline__ long long unit_place(const UnitList& L, int u, int lane, Unit& w) {
+// Lane `lane` of unit u of the list: everything but the quartet itself, which
+// is at `at` of the quartet buffer; false past the end.  The lanes without a
+// quartet (the tail of a sub-class) repeat the sub-class's last one and do
+// not store.
+__device__ __forceinline__ bool unit_place(const UnitList& L, int u, int lane, Unit& w, long long& at) {
     const int p = L.prec;
-    if (u >= L.nunit[2 * L.cls + p]) return -1;
+    if (u >= L.nunit[2 * L.cls + p]) return false;
     int lo = L.sub0, hi = L.sub1 - 1;  // last sub-class whose first unit is <= u
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -70,14 +70,14 @@ __device__ __forceinline__ long long unit_place(const UnitList& L, int u, int la
     }
     const ScreenSub& S = L.subs[lo];
     const int lgb = S.lgb[p], lgk = S.lgk[p], lg = lgb + lgk;
-    const long long n = (long long)L.cnt[2 * lo + p];
-    const long long i = ((long long)(u - S.unit[p]) << (5 - lg)) + (lane >> lg);
+    const long long first = (long long)(u - S.unit[p]) << (5 - lg);  // within the sub-class
+    const long long rest = (long long)L.cnt[2 * lo + p] - first;
+    const int n = (int)(rest < 32 ? rest : 32), i = lane >> lg;  // of this unit
     const int g = lane & ((1 << lg) - 1);
-    const long long at = S.off[p] + (i < n ? i : n - 1);
-    w.t = at - list_start(L);
+    at = S.off[p] + first + (i < n ? i : n - 1);
     w.store = i < n && g == 0;
     w.ls = LaneSplit{g >> lgk, 1 << lgb, g & ((1 << lgk) - 1), 1 << lgk, 1 << lg};
-    return at;
+    return true;
 }
 
 // The units [u0, u1) that hold entries [first, first + n) of the quartet

@@ -82,10 +82,10 @@ int hl_unit(const long long* cnt, const long long* off, const int* unit, const i
     Lists x = make(cnt, off, unit, lgb, lgk, nsub, nunit, coff, prec, n64);
     for (int lane = 0; lane < 32; ++lane) {
         Unit w;
-        const long long at = unit_place(x.L, u, lane, w);
-        if (at < 0) return 0;
+        long long at;
+        if (!unit_place(x.L, u, lane, w, at)) return 0;
         out[3 * lane] = at;
-        out[3 * lane + 1] = w.t;
+        out[3 * lane + 1] = at - list_start(x.L);
         out[3 * lane + 2] = w.store;
     }
     return 1;
